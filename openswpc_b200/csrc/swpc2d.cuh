@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "swpc_ctx.h"
+#include "swpc_kernels.cuh"
 
 namespace swpc {
 
@@ -46,6 +47,19 @@ struct Wav2Args {
     float M0, UC, dt;
 };
 
+// What a staged launch of a time step also does (all zero: nothing): the
+// stress launch adds the sources of its cells (inj, one per model) and records
+// in its first nwav CTAs the nlist recorders; the velocity
+// launch moves the counter it_next on (nothing of it reads the counter).
+struct Step2D {
+    const StepInj *inj;
+    const Wav2Args *wav;
+    int nlist, nwav;
+    int it;
+    const int *d_it;
+    int *it_next;
+};
+
 // Launch shape of the tile kernels: tiles of 32 (k) x (ti * ri) (i) cells,
 // one block of 32 x ti threads per tile with ri rows per thread, and a
 // persistent grid of 148 x blocks_per_sm blocks (0: one block per tile).
@@ -81,9 +95,10 @@ bool encode_maps2d(Maps2D &m, int kind, int nm, float *slab, const Geo &g);
 // model0 + nset - 1 (nset = 1 .. kGroup2D), whose map sets are sets[0 .. nset-1]
 cudaError_t launch_stress2d_tma(int kind, int nm, int ti, const MapSet2D *sets, int nset, int model0,
                                 const Model2D *models, const Tile2D *tiles, int ntiles, int mask, Fields2D f, int *err,
-                                cudaStream_t st);
+                                cudaStream_t st, const Step2D &x = Step2D());
 cudaError_t launch_vel2d_tma(int kind, int ti, const MapSet2D *sets, int nset, int model0, const Model2D *models,
-                             const Tile2D *tiles, int ntiles, int mask, Fields2D f, int *err, cudaStream_t st);
+                             const Tile2D *tiles, int ntiles, int mask, Fields2D f, int *err, cudaStream_t st,
+                             const Step2D &x = Step2D());
 // flags of the tile (k0, i0) of a model (tile extents 32 x ni)
 int tile2d_flags(const swpc_ctx *c, int k0, int i0, int ni);
 

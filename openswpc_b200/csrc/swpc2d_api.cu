@@ -74,6 +74,7 @@ int create_2d(swpc_ctx *c) {
     if (!rc) rc = dalloc(c, &c->kfs, g.Ip);
     if (!rc) rc = dalloc(c, &c->d_model2d, 1);
     if (!rc) rc = dalloc(c, &c->d_wav2d, 1);
+    if (!rc) rc = dalloc(c, &c->d_inj2d, 1);
     if (!rc) rc = dalloc(c, &c->d_err, 1);
     c->nm2d_aux = psv ? 8 : 4;
     if (rc) return rc;
@@ -183,6 +184,7 @@ void destroy_2d(swpc_ctx *c) {
     c->maps2d = nullptr;
     if (c->d_tiles2d) cudaFree(c->d_tiles2d);
     if (c->d_wav2d) cudaFree(c->d_wav2d);
+    if (c->d_inj2d) cudaFree(c->d_inj2d);
     if (c->rho_cell_bf) cudaFree(c->rho_cell_bf);
 }
 
@@ -285,45 +287,45 @@ Model2D model_of(const swpc_ctx *c) {
     return m;
 }
 
-int update_stress_2d_kernel(swpc_ctx *c, int mask);
-int update_vel_2d_kernel(swpc_ctx *c, int mask);
+int update_stress_2d_kernel(swpc_ctx *c, int mask, const Step2D &x = Step2D());
+int update_vel_2d_kernel(swpc_ctx *c, int mask, const Step2D &x = Step2D());
 
-int update_stress_2d(swpc_ctx *c, int mask) {
+int update_stress_2d(swpc_ctx *c, int mask, const Step2D &x) {
     if (c->abc == 1) {
         // Cerjan: the interior update over the whole domain, then the sponge
         if (mask & 1) RC(update_stress_2d_kernel(c, 1));
         if (mask & 2) RC(launch_cerjan2d(c, 0, c->stream));
         return SWPC_OK;
     }
-    return update_stress_2d_kernel(c, mask);
+    return update_stress_2d_kernel(c, mask, x);
 }
 
-int update_stress_2d_kernel(swpc_ctx *c, int mask) {
+int update_stress_2d_kernel(swpc_ctx *c, int mask, const Step2D &x) {
     const int m = (c->d.na > 0 && c->abc == 0) ? mask : (mask & 1);
     if (c->stress_tma)
         return cuda_check(c, launch_stress2d_tma(c->kind, c->d.nm, c->stress_tbi, &static_cast<Maps2D *>(c->maps2d)->str,
                                                  1, 0, c->d_model2d, c->d_tiles2d, c->ntiles2d, m,
-                                                 fields2d(c->kind, c->d.nm), c->d_err, c->stream),
+                                                 fields2d(c->kind, c->d.nm), c->d_err, c->stream, x),
                           "stress2d_tma launch");
     launch_stress2d(c->kind, c->d.nm, c->d_model2d, c->d_tiles2d, c->ntiles2d, m, kDefaultTiles, c->stream);
     return cuda_check(c, cudaGetLastError(), "stress2d launch");
 }
 
-int update_vel_2d(swpc_ctx *c, int mask) {
+int update_vel_2d(swpc_ctx *c, int mask, const Step2D &x) {
     if (c->abc == 1) {
         if (mask & 1) RC(update_vel_2d_kernel(c, 1));
         if (mask & 2) RC(launch_cerjan2d(c, 1, c->stream));
         return SWPC_OK;
     }
-    return update_vel_2d_kernel(c, mask);
+    return update_vel_2d_kernel(c, mask, x);
 }
 
-int update_vel_2d_kernel(swpc_ctx *c, int mask) {
+int update_vel_2d_kernel(swpc_ctx *c, int mask, const Step2D &x) {
     const int m = (c->d.na > 0 && c->abc == 0) ? mask : (mask & 1);
     if (c->vel_tma)
         return cuda_check(c, launch_vel2d_tma(c->kind, c->vel_tbi, &static_cast<Maps2D *>(c->maps2d)->vel, 1, 0,
                                               c->d_model2d, c->d_tiles2d, c->ntiles2d, m, fields2d(c->kind, c->d.nm),
-                                              c->d_err, c->stream),
+                                              c->d_err, c->stream, x),
                           "vel2d_tma launch");
     launch_vel2d(c->kind, c->d_model2d, c->d_tiles2d, c->ntiles2d, m, kDefaultTiles, c->stream);
     return cuda_check(c, cudaGetLastError(), "vel2d launch");
@@ -342,6 +344,12 @@ Wav2Args wav_of(const swpc_ctx *c) {
     return a;
 }
 
+// the stress-glut sources of a model as the staged stress launch adds them
+StepInj inj_of(const swpc_ctx *c) {
+    if (c->ninj_glut <= 0 || !c->glut_cols.list) return StepInj{};
+    return StepInj{c->glut_cols.col, c->glut_cols.list, c->stime_glut, c->mo_glut, c->nsrc_glut, c->d.nt, c->dt_dxyz};
+}
+
 int wav_store_2d(swpc_ctx *c, int it, const int *d_it) {
     launch_wav2d(c->d_wav2d, 1, c->nst, it, d_it, c->stream);
     return cuda_check(c, cudaGetLastError(), "wav2d launch");
@@ -353,6 +361,8 @@ int refresh_2d(swpc_ctx *c) {
     if (!c->desc_dirty) return SWPC_OK;
     const Model2D m = model_of(c);
     const Wav2Args w = wav_of(c);
+    const StepInj j = inj_of(c);
+    CK(cudaMemcpyAsync(c->d_inj2d, &j, sizeof(j), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(c->d_model2d, &m, sizeof(m), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(c->d_wav2d, &w, sizeof(w), cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -394,6 +404,10 @@ struct swpc_batch {
     int max_nst = 0;
     InjArgs *d_inj = nullptr;
     int ninj = 0, max_inj = 0;
+    // the members' stress-glut sources as the staged stress launches add them
+    // (null: a member runs the sponge, or its list has no such form)
+    StepInj *d_stepinj = nullptr;
+    int nwavlist = 0;   // recorders in d_wav
     int *d_it = nullptr;
     cudaGraphExec_t graph = nullptr;
     bool psv_bf_split = false;
@@ -427,7 +441,7 @@ extern "C" int swpc_batch_destroy(swpc_batch *b) {
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->graph) cudaGraphExecDestroy(b->graph);
-    void *ps[] = {b->d_models, b->d_tiles, b->d_wav, b->d_inj, b->d_it, b->d_err};
+    void *ps[] = {b->d_models, b->d_tiles, b->d_wav, b->d_inj, b->d_it, b->d_err, b->d_stepinj};
     for (void *p : ps) if (p) cudaFree(p);
     delete b;
     return SWPC_OK;
@@ -522,6 +536,19 @@ extern "C" int swpc_batch_create(swpc_ctx *const *members, int n, swpc_batch **o
     BCK(cudaMemcpy(b->d_models, models.data(), models.size() * sizeof(Model2D), cudaMemcpyHostToDevice));
     if (!wavs.empty()) BCK(cudaMemcpy(b->d_wav, wavs.data(), wavs.size() * sizeof(Wav2Args), cudaMemcpyHostToDevice));
     b->max_nst = wavs.empty() ? 0 : b->max_nst;
+    b->nwavlist = (int)wavs.size();
+    {
+        std::vector<StepInj> sj;
+        bool ok = true;
+        for (auto *c : b->members) {
+            sj.push_back(inj_of(c));
+            ok = ok && c->abc == 0 && (c->ninj_glut <= 0 || c->glut_cols.list);
+        }
+        if (ok) {
+            BCK(cudaMalloc(&b->d_stepinj, sj.size() * sizeof(StepInj)));
+            BCK(cudaMemcpy(b->d_stepinj, sj.data(), sj.size() * sizeof(StepInj), cudaMemcpyHostToDevice));
+        }
+    }
     // injection: stress glut lists then body-force lists of every member
     std::vector<InjArgs> glut, bf;
     for (auto *c : b->members) {
@@ -537,12 +564,16 @@ extern "C" int swpc_batch_create(swpc_ctx *const *members, int n, swpc_batch **o
     return SWPC_OK;
 }
 
-static int batch_step(swpc_batch *b, int it, const int *d_it) {
-    int nwav = 0, max_inj_n = 0;
-    for (auto *c : b->members) {
-        if (c->nst > 0 && c->wav_what) nwav++;
-        max_inj_n = std::max(max_inj_n, std::max(c->ninj_glut, c->ninj_bf));
-    }
+// *counted: the last velocity launch has moved the step counter of graph replays on
+static int batch_step(swpc_batch *b, int it, const int *d_it, bool *counted = nullptr) {
+    int max_inj_n = 0;
+    for (auto *c : b->members) max_inj_n = std::max(max_inj_n, std::max(c->ninj_glut, c->ninj_bf));
+    const int nwav = b->nwavlist;
+    // the staged launches take the recorders (the first group's), the sources
+    // and the counter (the last velocity launch) along (swpc_step.cuh)
+    const bool fuse_wav = b->sti && nwav > 0, fuse_src = b->sti && b->d_stepinj && b->ninj > 0;
+    const bool count = counted && d_it && b->vti && b->max_inj == 0;
+    if (count) *counted = true;
     const int mask_all = 3;
     const Fields2D f = fields2d(b->kind, b->nm);
     // staged: one launch per member group over that group's tiles
@@ -555,9 +586,18 @@ static int batch_step(swpc_batch *b, int it, const int *d_it) {
         for (int g = 0; g < ng; g++) {
             const int m0 = b->group_first[g], m1 = b->group_first[g + 1];
             const int t0 = b->tile_first[m0], t1 = b->tile_first[m1];
+            Step2D x = {};
+            x.it = it;
+            x.d_it = d_it;
+            if (fuse_src) x.inj = b->d_stepinj;
+            if (fuse_wav && g == 0) {
+                x.wav = b->d_wav;
+                x.nlist = nwav;
+                x.nwav = nwav * ((b->max_nst + kWavPerCta - 1) / kWavPerCta);
+            }
             const cudaError_t e = launch_stress2d_tma(b->kind, b->nm, b->sti, &b->str_sets[m0], m1 - m0, m0,
                                                       b->d_models, b->d_tiles + t0, t1 - t0, mask, f, b->d_err,
-                                                      b->stream);
+                                                      b->stream, x);
             if (e != cudaSuccess) return e;
         }
         return cudaSuccess;
@@ -570,8 +610,10 @@ static int batch_step(swpc_batch *b, int it, const int *d_it) {
         for (int g = 0; g < ng; g++) {
             const int m0 = b->group_first[g], m1 = b->group_first[g + 1];
             const int t0 = b->tile_first[m0], t1 = b->tile_first[m1];
+            Step2D x = {};
+            if (count && g == ng - 1) x.it_next = b->d_it;
             const cudaError_t e = launch_vel2d_tma(b->kind, b->vti, &b->vel_sets[m0], m1 - m0, m0, b->d_models,
-                                                   b->d_tiles + t0, t1 - t0, mask, f, b->d_err, b->stream);
+                                                   b->d_tiles + t0, t1 - t0, mask, f, b->d_err, b->stream, x);
             if (e != cudaSuccess) return e;
         }
         return cudaSuccess;
@@ -586,10 +628,10 @@ static int batch_step(swpc_batch *b, int it, const int *d_it) {
             }
         return (int)SWPC_OK;
     };
-    launch_wav2d(b->d_wav, nwav, b->max_nst, it, d_it, b->stream);
+    if (!fuse_wav) launch_wav2d(b->d_wav, nwav, b->max_nst, it, d_it, b->stream);
     BCK(stress(mask_all));
     RC(sponge(0));
-    launch_inject_multi(b->d_inj, b->ninj, max_inj_n, d_it, it, b->stream);
+    if (!fuse_src) launch_inject_multi(b->d_inj, b->ninj, max_inj_n, d_it, it, b->stream);
     if (b->kind == SWPC_KIND_PSV && b->psv_bf_split) {
         // P-SV applies body forces between the interior and absorber velocity
         // updates (src/swpc_psv/main.f90:106-110)
@@ -621,8 +663,9 @@ extern "C" int swpc_batch_run(swpc_batch *b, int it0, int nsteps) {
     if (!b->graph) {
         cudaGraph_t g;
         BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-        int rc = batch_step(b, 0, b->d_it);
-        if (!rc) launch_advance_it(b->d_it, b->stream);
+        bool counted = false;
+        int rc = batch_step(b, 0, b->d_it, &counted);
+        if (!rc && !counted) launch_advance_it(b->d_it, b->stream);
         cudaError_t e = cudaStreamEndCapture(b->stream, &g);
         if (rc) return rc;
         BCK(e);

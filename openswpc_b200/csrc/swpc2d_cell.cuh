@@ -276,4 +276,42 @@ __device__ __forceinline__ void sh_vel_cell(const Model2D &M, const O &o, int k,
     st2s(&azSyz[q], gzc.z * vzSyz + gzc.w * dzSyz * dt);
 }
 
+// ---------------------------------------------------------------------------
+// recorder: station n of one model (src/swpc_psv/m_wav.f90, src/swpc_sh/m_wav.f90)
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void wav2_station(const Wav2Args &a, int n, int it) {
+    const int i = a.st[2 * n], k = a.st[2 * n + 1];
+    const long long PI = a.Kp;
+    const long long e = (long long)(i + 2) * PI + (k - 1 + KH);
+    const float dt = a.dt;
+    if (a.what & SWPC_WAV_U) {
+        if (a.psv) {
+            a.uacc[2 * n] = a.uacc[2 * n] + (a.V0[e] + a.V0[e - PI]) * 0.5f * dt;
+            a.uacc[2 * n + 1] = a.uacc[2 * n + 1] - (a.V1[e] + a.V1[e - 1]) * 0.5f * dt;
+        } else {
+            a.uacc[2 * n] = a.uacc[2 * n] + a.V0[e] * dt;
+        }
+    }
+    if (it < 1 || (it - 1) % a.ntdec_w != 0) return;
+    const int itw = (it - 1) / a.ntdec_w + 1;
+    if (itw > a.ntw) return;
+    const long long ntw = a.ntw;
+    const int nc = a.psv ? 2 : 1;
+    const float M0 = a.M0, UC = a.UC;
+    if (a.what & SWPC_WAV_V) {
+        float *w = a.wav_v + (long long)n * nc * ntw + (itw - 1);
+        if (a.psv) {
+            w[0] = (a.V0[e] + a.V0[e - PI]) / 2.0f * M0 * UC * 1e9f;
+            w[ntw] = -(a.V1[e] + a.V1[e - 1]) / 2.0f * M0 * UC * 1e9f;
+        } else {
+            w[0] = a.V0[e] * M0 * UC * 1e9f;
+        }
+    }
+    if (a.what & SWPC_WAV_U) {
+        float *w = a.wav_u + (long long)n * nc * ntw + (itw - 1);
+        w[0] = a.uacc[2 * n] * M0 * UC * 1e9f;
+        if (a.psv) w[ntw] = a.uacc[2 * n + 1] * M0 * UC * 1e9f;
+    }
+}
+
 }  // namespace swpc

@@ -81,43 +81,9 @@ __global__ void __launch_bounds__(256) tile2d_kernel(const Model2D *__restrict__
 // ---------------------------------------------------------------------------
 __global__ void wav2d_kernel(const Wav2Args *__restrict__ list, int nlist, int it_arg, const int *d_it) {
     const int it = d_it ? *d_it : it_arg;
-    for (int b = blockIdx.y; b < nlist; b += gridDim.y) {
-        const Wav2Args &a = list[b];
-        for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < a.nst; n += gridDim.x * blockDim.x) {
-            const int i = a.st[2 * n], k = a.st[2 * n + 1];
-            const long long PI = a.Kp;
-            const long long e = (long long)(i + 2) * PI + (k - 1 + KH);
-            const float dt = a.dt;
-            if (a.what & SWPC_WAV_U) {
-                if (a.psv) {
-                    a.uacc[2 * n] = a.uacc[2 * n] + (a.V0[e] + a.V0[e - PI]) * 0.5f * dt;
-                    a.uacc[2 * n + 1] = a.uacc[2 * n + 1] - (a.V1[e] + a.V1[e - 1]) * 0.5f * dt;
-                } else {
-                    a.uacc[2 * n] = a.uacc[2 * n] + a.V0[e] * dt;
-                }
-            }
-            if (it < 1 || (it - 1) % a.ntdec_w != 0) continue;
-            const int itw = (it - 1) / a.ntdec_w + 1;
-            if (itw > a.ntw) continue;
-            const long long ntw = a.ntw;
-            const int nc = a.psv ? 2 : 1;
-            const float M0 = a.M0, UC = a.UC;
-            if (a.what & SWPC_WAV_V) {
-                float *w = a.wav_v + (long long)n * nc * ntw + (itw - 1);
-                if (a.psv) {
-                    w[0] = (a.V0[e] + a.V0[e - PI]) / 2.0f * M0 * UC * 1e9f;
-                    w[ntw] = -(a.V1[e] + a.V1[e - 1]) / 2.0f * M0 * UC * 1e9f;
-                } else {
-                    w[0] = a.V0[e] * M0 * UC * 1e9f;
-                }
-            }
-            if (a.what & SWPC_WAV_U) {
-                float *w = a.wav_u + (long long)n * nc * ntw + (itw - 1);
-                w[0] = a.uacc[2 * n] * M0 * UC * 1e9f;
-                if (a.psv) w[ntw] = a.uacc[2 * n + 1] * M0 * UC * 1e9f;
-            }
-        }
-    }
+    for (int b = blockIdx.y; b < nlist; b += gridDim.y)
+        for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < list[b].nst; n += gridDim.x * blockDim.x)
+            wav2_station(list[b], n, it);
 }
 
 __global__ void vmax2d_kernel(const float *V0, const float *V1, const int *kob, int Kp, int i0, int i1,

@@ -33,6 +33,7 @@
 
 #include "swpc2d.cuh"
 #include "swpc2d_cell.cuh"
+#include "swpc_step.cuh"
 #include "swpc_tma_ptx.cuh"
 
 namespace swpc {
@@ -140,11 +141,19 @@ struct SVel2 {
 // ---------------------------------------------------------------------------
 // kernels
 // ---------------------------------------------------------------------------
+// the recorder's CTAs of a stress launch: kWavPerCta stations of one list entry
+__device__ __noinline__ void record(const Step2D &x, int cta) {
+    const Wav2Args &w = x.wav[cta % x.nlist];
+    const int t = threadIdx.y * blockDim.x + threadIdx.x, n = cta / x.nlist * kWavPerCta + t;
+    if (t < kWavPerCta && n < w.nst) wav2_station(w, n, x.d_it ? *x.d_it : x.it);
+}
+
 template <int KIND, int NM, int TI, int G>
 __global__ void __launch_bounds__(32 * TI) stress2d_tma_kernel(const __grid_constant__ MapGroup<G> pm, int model0,
                                                                const Model2D *__restrict__ models,
                                                                const Tile2D *__restrict__ tiles, int mask,
-                                                               Fields2D f, int *err) {
+                                                               Fields2D f, int *err,
+                                                               const __grid_constant__ Step2D x) {
     using L = StrBox<KIND, NM>;
     constexpr int RI = BI / TI;
     extern __shared__ __align__(128) unsigned char smraw[];
@@ -152,15 +161,25 @@ __global__ void __launch_bounds__(32 * TI) stress2d_tma_kernel(const __grid_cons
     __shared__ __align__(8) uint64_t bar;
     __shared__ unsigned long long limit;
     float *sm = aligned128(smraw);
-    const Tile2D tl = tiles[blockIdx.x];
+    if (blockIdx.x < x.nwav) {
+        pdl_wait();
+        pdl_launch();
+        record(x, blockIdx.x);
+        return;
+    }
+    const Tile2D tl = tiles[blockIdx.x - x.nwav];
     const int tx = threadIdx.x, ty = threadIdx.y;
     const bool lead = tx == 0 && ty == 0;
     // interior cells need S, R and the medium, absorber cells S and the medium
     const bool with_r = (mask & 1) && (tl.flags & kTileInterior);
-    if (!with_r && !((mask & 2) && (tl.flags & kTileAbsorber))) return;   // nothing of this launch here
+    if (!with_r && !((mask & 2) && (tl.flags & kTileAbsorber))) {   // nothing of this launch here
+        pdl_wait();   // a launch ends after the one before it
+        return;
+    }
     if (lead) {
         // the copies go out first; the error word is read while they travel
         stage_init(&bar, L::bytes(with_r));
+        pdl_wait();
         const CUtensorMap *mp = set_maps(pm.set[tl.model - model0]);
         const int x0 = tl.k0 - 1 + KH, ic = tl.i0 + 2;
         load_3d(sm + L::oState, with_r ? &mp[ST_STATE] : &mp[ST_S], x0, ic, f.s, &bar);
@@ -170,15 +189,19 @@ __global__ void __launch_bounds__(32 * TI) stress2d_tma_kernel(const __grid_cons
         limit = wait_limit(err);
     }
     copy_model(models, tl.model, sM);
+    pdl_wait();
+    pdl_launch();
     __syncthreads();   // barrier initialised, wait limit and model descriptor set
     const Model2D &M = sM;
-    // the band signs of this thread's cells are read while the tiles travel
-    int sg[RI];
+    // the band signs and source columns of this thread's cells are read while the tiles travel
+    const int *icol = x.inj ? x.inj[tl.model].col : nullptr;
+    int sg[RI], src[RI];
 #pragma unroll
     for (int r = 0; r < RI; r++) {
         const int k = tl.k0 + tx, i = tl.i0 + ty + r * TI;
         const bool interior = i >= M.ibk && i <= M.iek && k <= M.kek;
         sg[r] = (interior && k <= M.nz && (mask & 1)) ? band_sign2d(M, k, i) : -1;
+        src[r] = (icol && i <= M.nx) ? __ldg(&icol[i + 2]) : -1;
     }
     if (!wait_tiles(&bar, err, limit)) return;   // the copy did not complete
 #pragma unroll
@@ -197,6 +220,7 @@ __global__ void __launch_bounds__(32 * TI) stress2d_tma_kernel(const __grid_cons
         } else {
             sh_stress_cell<NM>(M, o, k, i, e, s);
         }
+        if (src[r] >= 0) inject_cell(x.inj[tl.model], x.d_it ? *x.d_it : x.it, src[r], e);
     }
 }
 
@@ -204,7 +228,7 @@ template <int KIND, int TI, int G>
 __global__ void __launch_bounds__(32 * TI) vel2d_tma_kernel(const __grid_constant__ MapGroup<G> pm, int model0,
                                                             const Model2D *__restrict__ models,
                                                             const Tile2D *__restrict__ tiles, int mask, Fields2D f,
-                                                            int *err) {
+                                                            int *err, int *it_next) {
     using L = VelBox<KIND>;
     constexpr int RI = BI / TI;
     extern __shared__ __align__(128) unsigned char smraw[];
@@ -215,10 +239,18 @@ __global__ void __launch_bounds__(32 * TI) vel2d_tma_kernel(const __grid_constan
     const Tile2D tl = tiles[blockIdx.x];
     const int tx = threadIdx.x, ty = threadIdx.y;
     const bool lead = tx == 0 && ty == 0;
-    if (!((mask & 1) && (tl.flags & kTileInterior)) && !((mask & 2) && (tl.flags & kTileAbsorber))) return;
+    if (it_next && lead && blockIdx.x == 0) {
+        pdl_wait();
+        *it_next = *it_next + 1;   // no other CTA of this launch reads it
+    }
+    if (!((mask & 1) && (tl.flags & kTileInterior)) && !((mask & 2) && (tl.flags & kTileAbsorber))) {
+        pdl_wait();   // a launch ends after the one before it
+        return;
+    }
     if (lead) {
         // the copies go out first; the error word is read while they travel
         stage_init(&bar, L::bytes());
+        pdl_wait();
         const CUtensorMap *mp = set_maps(pm.set[tl.model - model0]);
         const int x0 = tl.k0 - 1 + KH, ic = tl.i0 + 2;
         load_3d(sm + L::oOwn, &mp[VE_OWN], x0, ic, f.v, &bar);
@@ -234,6 +266,8 @@ __global__ void __launch_bounds__(32 * TI) vel2d_tma_kernel(const __grid_constan
         limit = wait_limit(err);
     }
     copy_model(models, tl.model, sM);
+    pdl_wait();
+    pdl_launch();
     __syncthreads();   // barrier initialised, wait limit and model descriptor set
     const Model2D &M = sM;
     // the band signs of this thread's cells are read while the tiles travel
@@ -287,67 +321,65 @@ MapGroup<G> group_of(const MapArgs &ma) {
 
 template <int KIND, int NM, int TI, int G>
 cudaError_t run_stress(const MapArgs &ma, const Model2D *models, const Tile2D *tiles, int ntiles, int mask,
-                       Fields2D f, int *err, cudaStream_t st) {
+                       Fields2D f, int *err, cudaStream_t st, const Step2D &x) {
     constexpr int bytes = StrBox<KIND, NM>::total * 4 + 128;
     static unsigned long long devices = 0;
     cudaError_t e = smem_attr(stress2d_tma_kernel<KIND, NM, TI, G>, bytes, devices);
     if (e != cudaSuccess) return e;
-    stress2d_tma_kernel<KIND, NM, TI, G><<<ntiles, dim3(32, TI), bytes, st>>>(group_of<G>(ma), ma.model0, models, tiles,
-                                                                              mask, f, err);
-    return cudaGetLastError();
+    return launch_pdl(stress2d_tma_kernel<KIND, NM, TI, G>, dim3(ntiles + x.nwav), dim3(32, TI), bytes, st,
+                      group_of<G>(ma), ma.model0, models, tiles, mask, f, err, x);
 }
 
 template <int KIND, int TI, int G>
 cudaError_t run_vel(const MapArgs &ma, const Model2D *models, const Tile2D *tiles, int ntiles, int mask,
-                    Fields2D f, int *err, cudaStream_t st) {
+                    Fields2D f, int *err, cudaStream_t st, const Step2D &x) {
     constexpr int bytes = VelBox<KIND>::total * 4 + 128;
     static unsigned long long devices = 0;
     cudaError_t e = smem_attr(vel2d_tma_kernel<KIND, TI, G>, bytes, devices);
     if (e != cudaSuccess) return e;
-    vel2d_tma_kernel<KIND, TI, G><<<ntiles, dim3(32, TI), bytes, st>>>(group_of<G>(ma), ma.model0, models, tiles, mask,
-                                                                       f, err);
-    return cudaGetLastError();
+    return launch_pdl(vel2d_tma_kernel<KIND, TI, G>, dim3(ntiles), dim3(32, TI), bytes, st, group_of<G>(ma), ma.model0,
+                      models, tiles, mask, f, err, x.it_next);
 }
 
 template <int KIND, int NM, int TI>
 cudaError_t stress_g(const MapArgs &ma, const Model2D *models, const Tile2D *tiles, int ntiles, int mask, Fields2D f,
-                     int *err, cudaStream_t st) {
-    if (ma.nset > 1) return run_stress<KIND, NM, TI, kGroup2D>(ma, models, tiles, ntiles, mask, f, err, st);
-    return run_stress<KIND, NM, TI, 1>(ma, models, tiles, ntiles, mask, f, err, st);
+                     int *err, cudaStream_t st, const Step2D &x) {
+    if (ma.nset > 1) return run_stress<KIND, NM, TI, kGroup2D>(ma, models, tiles, ntiles, mask, f, err, st, x);
+    return run_stress<KIND, NM, TI, 1>(ma, models, tiles, ntiles, mask, f, err, st, x);
 }
 
 template <int KIND, int NM>
 cudaError_t stress_ti(int ti, const MapArgs &ma, const Model2D *models, const Tile2D *tiles, int ntiles, int mask,
-                      Fields2D f, int *err, cudaStream_t st) {
-    if (ti == 4) return stress_g<KIND, NM, 4>(ma, models, tiles, ntiles, mask, f, err, st);
-    if (ti == 16) return stress_g<KIND, NM, 16>(ma, models, tiles, ntiles, mask, f, err, st);
-    return stress_g<KIND, NM, 8>(ma, models, tiles, ntiles, mask, f, err, st);
+                      Fields2D f, int *err, cudaStream_t st, const Step2D &x) {
+    if (ti == 4) return stress_g<KIND, NM, 4>(ma, models, tiles, ntiles, mask, f, err, st, x);
+    if (ti == 16) return stress_g<KIND, NM, 16>(ma, models, tiles, ntiles, mask, f, err, st, x);
+    return stress_g<KIND, NM, 8>(ma, models, tiles, ntiles, mask, f, err, st, x);
 }
 
 template <int KIND>
 cudaError_t stress_nm(int nm, int ti, const MapArgs &ma, const Model2D *models, const Tile2D *tiles, int ntiles,
-                      int mask, Fields2D f, int *err, cudaStream_t st) {
+                      int mask, Fields2D f, int *err, cudaStream_t st, const Step2D &x) {
     switch (nm) {
-    case 0: return stress_ti<KIND, 0>(ti, ma, models, tiles, ntiles, mask, f, err, st);
-    case 1: return stress_ti<KIND, 1>(ti, ma, models, tiles, ntiles, mask, f, err, st);
-    case 2: return stress_ti<KIND, 2>(ti, ma, models, tiles, ntiles, mask, f, err, st);
-    default: return stress_ti<KIND, 3>(ti, ma, models, tiles, ntiles, mask, f, err, st);
+    case 0: return stress_ti<KIND, 0>(ti, ma, models, tiles, ntiles, mask, f, err, st, x);
+    case 1: return stress_ti<KIND, 1>(ti, ma, models, tiles, ntiles, mask, f, err, st, x);
+    case 2: return stress_ti<KIND, 2>(ti, ma, models, tiles, ntiles, mask, f, err, st, x);
+    default: return stress_ti<KIND, 3>(ti, ma, models, tiles, ntiles, mask, f, err, st, x);
     }
 }
 
 template <int KIND, int TI>
 cudaError_t vel_g(const MapArgs &ma, const Model2D *models, const Tile2D *tiles, int ntiles, int mask, Fields2D f,
-                  int *err, cudaStream_t st) {
-    if (ma.nset > 1) return run_vel<KIND, TI, kGroup2D>(ma, models, tiles, ntiles, mask, f, err, st);
-    return run_vel<KIND, TI, 1>(ma, models, tiles, ntiles, mask, f, err, st);
+                  int *err, cudaStream_t st, const Step2D &x) {
+    if (ma.nset > 1) return run_vel<KIND, TI, kGroup2D>(ma, models, tiles, ntiles, mask, f, err, st, x);
+    return run_vel<KIND, TI, 1>(ma, models, tiles, ntiles, mask, f, err, st, x);
 }
 
 template <int KIND>
 cudaError_t vel_ti(int ti, const MapArgs &ma, const Model2D *models, const Tile2D *tiles, int ntiles, int mask,
-                   Fields2D f, int *err, cudaStream_t st) {
-    if (ti == 4) return vel_g<KIND, 4>(ma, models, tiles, ntiles, mask, f, err, st);
-    if (ti == 16) return vel_g<KIND, 16>(ma, models, tiles, ntiles, mask, f, err, st);
-    return vel_g<KIND, 8>(ma, models, tiles, ntiles, mask, f, err, st);
+                   Fields2D f, int *err, cudaStream_t st, const Step2D &x) {
+    if (ti == 4) return vel_g<KIND, 4>(ma, models, tiles, ntiles, mask, f, err, st, x);
+    if (ti == 16) return vel_g<KIND, 16>(ma, models, tiles, ntiles, mask, f, err, st, x);
+    return vel_g<KIND, 8>(ma, models, tiles, ntiles, mask, f, err, st, x);
 }
 
 // 3D map (k, i, field) over a model's slab with the given box; L2 fills of
@@ -406,21 +438,21 @@ bool encode_maps2d(Maps2D &m, int kind, int nm, float *slab, const Geo &g) {
 
 cudaError_t launch_stress2d_tma(int kind, int nm, int ti, const MapSet2D *sets, int nset, int model0,
                                 const Model2D *models, const Tile2D *tiles, int ntiles, int mask, Fields2D f, int *err,
-                                cudaStream_t st) {
+                                cudaStream_t st, const Step2D &x) {
     if (ntiles <= 0) return cudaSuccess;
     if (nset < 1 || nset > kGroup2D) return cudaErrorInvalidValue;
     const MapArgs ma{sets, nset, model0};
-    if (kind == SWPC_KIND_PSV) return stress_nm<0>(nm, ti, ma, models, tiles, ntiles, mask, f, err, st);
-    return stress_nm<1>(nm, ti, ma, models, tiles, ntiles, mask, f, err, st);
+    if (kind == SWPC_KIND_PSV) return stress_nm<0>(nm, ti, ma, models, tiles, ntiles, mask, f, err, st, x);
+    return stress_nm<1>(nm, ti, ma, models, tiles, ntiles, mask, f, err, st, x);
 }
 
 cudaError_t launch_vel2d_tma(int kind, int ti, const MapSet2D *sets, int nset, int model0, const Model2D *models,
-                             const Tile2D *tiles, int ntiles, int mask, Fields2D f, int *err, cudaStream_t st) {
+                             const Tile2D *tiles, int ntiles, int mask, Fields2D f, int *err, cudaStream_t st, const Step2D &x) {
     if (ntiles <= 0) return cudaSuccess;
     if (nset < 1 || nset > kGroup2D) return cudaErrorInvalidValue;
     const MapArgs ma{sets, nset, model0};
-    if (kind == SWPC_KIND_PSV) return vel_ti<0>(ti, ma, models, tiles, ntiles, mask, f, err, st);
-    return vel_ti<1>(ti, ma, models, tiles, ntiles, mask, f, err, st);
+    if (kind == SWPC_KIND_PSV) return vel_ti<0>(ti, ma, models, tiles, ntiles, mask, f, err, st, x);
+    return vel_ti<1>(ti, ma, models, tiles, ntiles, mask, f, err, st, x);
 }
 
 }  // namespace swpc

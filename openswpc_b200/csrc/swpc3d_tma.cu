@@ -43,6 +43,7 @@
 #include <stdint.h>
 
 #include "swpc3d_cell.cuh"
+#include "swpc_step.cuh"
 #include "swpc_tma.h"
 #include "swpc_tma_ptx.cuh"
 #include "swpc_tma_tile.cuh"
@@ -110,6 +111,13 @@ struct SStrOps {
     __device__ __forceinline__ float med(int m) const { return sm[at(m == 0 ? 1 : m == 1 ? 0 : m)]; }
 };
 
+// the recorder's CTAs of a stress launch
+__device__ __noinline__ void record(const Wav3Args &w, int cta) {
+    const int t = (threadIdx.z * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
+    const int n = cta * kWavPerCta + t;
+    if (t < kWavPerCta && n < w.nst) wav_station(w, n);
+}
+
 // Maps by storage form: tm_state = S and R (F32 slab; F16_SR: the 2-byte
 // slab) or R alone (BF16_R: the 2-byte slab); tm_s = S alone (the slab that
 // holds S).
@@ -118,7 +126,8 @@ __global__ void __launch_bounds__(KT * BI * BJ,
                                   (blocks_per_sm<StrBoxes<NM, BI, BJ, M, PREC>::total, KT * BI * BJ>()))
     stress3d_tma_kernel(const __grid_constant__ CUtensorMap tm_state, const __grid_constant__ CUtensorMap tm_s,
                         const __grid_constant__ CUtensorMap tm_med, const __grid_constant__ CUtensorMap tm_v,
-                        const Str3Args a, const TmaTiles t) {
+                        const __grid_constant__ Str3Args a, const TmaTiles t,
+                        const __grid_constant__ StressExtra x) {
     static_assert(PREC == PREC_F32 || M == 1, "reduced storage forms run single members");
     using L = StrBoxes<NM, BI, BJ, M, PREC>;
     extern __shared__ __align__(128) unsigned char smraw[];
@@ -126,17 +135,31 @@ __global__ void __launch_bounds__(KT * BI * BJ,
     __shared__ unsigned long long limit;
     float *sm = aligned128(smraw);
     const Geo g = a.g;
-    const Tile T = tile_of<M>(t, BI, BJ);
+    if (blockIdx.x < x.nwav) {
+        pdl_wait();
+        pdl_launch();
+        record(x.wav, blockIdx.x);
+        return;
+    }
+    const Tile T = tile_of<M>(t, BI, BJ, blockIdx.x - x.nwav);
     const int tx = threadIdx.x, ty = threadIdx.y, tz = threadIdx.z;
     const bool lead = tx == 0 && ty == 0 && tz == 0;
+    if (x.it_copy && lead && blockIdx.x == x.nwav) {
+        pdl_wait();
+        *x.it_copy = *x.d_it;
+    }
     // cells of this launch in the tile: interior ones need S, R and the medium, absorber ones S and the medium
     const bool with_r = (a.mask & 1) && tile_has_interior(T, BI, BJ, a.ibk, a.iek, a.jbk, a.jek, a.kek);
     const bool staged =
         with_r || ((a.mask & 2) && tile_has_absorber(T, BI, BJ, g, a.ibk, a.iek, a.jbk, a.jek, a.kek));
-    if (!staged) return;   // nothing of this launch here (uniform over the CTA)
+    if (!staged) {   // nothing of this launch here (uniform over the CTA)
+        pdl_wait();  // a launch ends after the one before it
+        return;
+    }
     if (lead) {
         // the copies go out first; the error word is read while they travel
         stage_init(&bar, (unsigned)L::bytes(T.nmem, with_r));
+        pdl_wait();
         const int x0 = T.k0 - 1 + KH;
         load_4d(sm, &tm_med, x0, T.i0 + 2, T.j0 + 2, t.f_med, &bar);
         for (int mm = 0; mm < T.nmem; mm++) {
@@ -162,6 +185,9 @@ __global__ void __launch_bounds__(KT * BI * BJ,
     // the band sign of an interior cell and the auxiliaries of an absorber
     // cell (up to two members) are read while the tiles travel
     const int sgn = (mine && interior) ? band_sign_of(a.band, col, k) : 0;
+    const int src = (mine && x.inj.col) ? __ldg(&x.inj.col[col]) : -1;
+    pdl_wait();
+    pdl_launch();
     constexpr bool PRE = M <= 2;
     Aux9 xs[PRE ? M : 1];
     if (PRE && mine && !interior) {
@@ -181,10 +207,11 @@ __global__ void __launch_bounds__(KT * BI * BJ,
         if (interior) {
             stress_interior<NM, PREC>(a, o, sgn, Sp, e, so);
         } else {
-            const Aux9 x = PRE ? xs[PRE ? mm : 0] : aux_load(a.aV, ao, a.pmlcol, g, k, i, j);
-            stress_absorber<PREC>(a, o, x, k, i, j, e, ao, Sp);
+            const Aux9 ax = PRE ? xs[PRE ? mm : 0] : aux_load(a.aV, ao, a.pmlcol, g, k, i, j);
+            stress_absorber<PREC>(a, o, ax, k, i, j, e, ao, Sp);
         }
     }
+    if (src >= 0) inject_cell(x.inj, x.d_it ? *x.d_it : x.it, src, e);   // single members only
 }
 
 // ---------------------------------------------------------------------------
@@ -258,7 +285,8 @@ __global__ void __launch_bounds__(KT * BI, (blocks_per_sm<VelBoxes<BI, BJ, M, PR
                      const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_by,
                      const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ CUtensorMap tm_f,
                      const __grid_constant__ CUtensorMap tm_e, const __grid_constant__ CUtensorMap tm_d,
-                     const Vel3Args a, const TmaTiles t) {
+                     const __grid_constant__ Vel3Args a, const TmaTiles t,
+                     const __grid_constant__ VelExtra x) {
     static_assert(PREC == PREC_F32 || M == 1, "reduced storage forms run single members");
     using L = VelBoxes<BI, BJ, M, PREC>;
     extern __shared__ __align__(128) unsigned char smraw[];
@@ -266,15 +294,23 @@ __global__ void __launch_bounds__(KT * BI, (blocks_per_sm<VelBoxes<BI, BJ, M, PR
     __shared__ unsigned long long limit;
     float *sm = aligned128(smraw);
     const Geo g = a.g;
-    const Tile T = tile_of<M>(t, BI, BJ);
+    const Tile T = tile_of<M>(t, BI, BJ, blockIdx.x);
     const int tx = threadIdx.x, ty = threadIdx.y;
     const bool lead = tx == 0 && ty == 0;
+    if (x.it_next && lead && blockIdx.x == 0) {
+        pdl_wait();
+        *x.it_next = *x.it_next + 1;   // no other CTA of this launch reads it
+    }
     const bool staged = ((a.mask & 1) && tile_has_interior(T, BI, BJ, a.ibk, a.iek, a.jbk, a.jek, a.kek)) ||
                         ((a.mask & 2) && tile_has_absorber(T, BI, BJ, g, a.ibk, a.iek, a.jbk, a.jek, a.kek));
-    if (!staged) return;   // nothing of this launch here (uniform over the CTA)
+    if (!staged) {   // nothing of this launch here (uniform over the CTA)
+        pdl_wait();  // a launch ends after the one before it
+        return;
+    }
     if (lead) {
         // the copies go out first; the error word is read while they travel
         stage_init(&bar, (unsigned)L::bytes(T.nmem));
+        pdl_wait();
         const int x0 = T.k0 - 1 + KH, ic = T.i0 + 2, jc = T.j0 + 2;
         load_4d(sm, &tm_b, x0, ic, jc, t.f_b, &bar);
         for (int mm = 0; mm < T.nmem; mm++) {
@@ -296,13 +332,16 @@ __global__ void __launch_bounds__(KT * BI, (blocks_per_sm<VelBoxes<BI, BJ, M, PR
     // read while the tiles travel: the band signs of this thread's interior
     // cells, and the auxiliaries of its absorber cells (up to two cells: BJ
     // planes x M members)
-    int sgn[BJ];
+    int sgn[BJ], src[BJ];
 #pragma unroll
     for (int jj = 0; jj < BJ; jj++) {
         const int j = T.j0 + jj;
         const bool interior = i >= a.ibk && i <= a.iek && j >= a.jbk && j <= a.jek && k <= a.kek;
         sgn[jj] = (col_ok && interior && (a.mask & 1)) ? band_sign_of(a.band, col_index(g, i, j), k) : 0;
+        src[jj] = (x.inj.col && col_ok && j <= g.ny) ? __ldg(&x.inj.col[col_index(g, i, j)]) : -1;
     }
+    pdl_wait();
+    pdl_launch();
     constexpr bool PRE = BJ * M <= 2;
     Aux9 xs[PRE ? M : 1][PRE ? BJ : 1];
     if (PRE && col_ok && (a.mask & 2)) {
@@ -332,9 +371,10 @@ __global__ void __launch_bounds__(KT * BI, (blocks_per_sm<VelBoxes<BI, BJ, M, PR
             if (interior) {
                 vel_interior<PREC>(a, o, sgn[jj], a.Vx + so, a.Vy + so, a.Vz + so, e);
             } else {
-                const Aux9 x = PRE ? xs[PRE ? mm : 0][PRE ? jj : 0] : aux_load(a.aS, ao, a.pmlcol, g, k, i, j);
-                vel_absorber<PREC>(a, o, x, k, i, j, e, ao, a.Vx + so, a.Vy + so, a.Vz + so);
+                const Aux9 ax = PRE ? xs[PRE ? mm : 0][PRE ? jj : 0] : aux_load(a.aS, ao, a.pmlcol, g, k, i, j);
+                vel_absorber<PREC>(a, o, ax, k, i, j, e, ao, a.Vx + so, a.Vy + so, a.Vz + so);
             }
+            if (src[jj] >= 0) inject_cell(x.inj, x.d_it ? *x.d_it : x.it, src[jj], e);   // single members only
         }
     }
 }
@@ -352,37 +392,35 @@ cudaError_t smem_attr(K kernel, int bytes, unsigned long long &devices) {
 inline const CUtensorMap &map(const unsigned char *p) { return *reinterpret_cast<const CUtensorMap *>(p); }
 
 template <int NM, int BI, int BJ, int M, int PREC>
-cudaError_t run_stress(const TmaMaps &m, const Str3Args &a, const TmaTiles &t, cudaStream_t st) {
+cudaError_t run_stress(const TmaMaps &m, const Str3Args &a, const TmaTiles &t, const StressExtra &x, cudaStream_t st) {
     constexpr int bytes = StrBoxes<NM, BI, BJ, M, PREC>::total * 4 + 128;
     static unsigned long long devices = 0;   // devices on which the attribute is set
     cudaError_t e = smem_attr(stress3d_tma_kernel<NM, BI, BJ, M, PREC>, bytes, devices);
     if (e != cudaSuccess) return e;
     const unsigned nblk = (unsigned)((long long)t.nkt * t.nit * t.njt * t.mgroups);
-    stress3d_tma_kernel<NM, BI, BJ, M, PREC><<<nblk, dim3(KT, BI, BJ), bytes, st>>>(map(m.state), map(m.s6),
-                                                                                     map(m.med), map(m.vh), a, t);
-    return cudaGetLastError();
+    return launch_pdl(stress3d_tma_kernel<NM, BI, BJ, M, PREC>, dim3(nblk + x.nwav), dim3(KT, BI, BJ), bytes, st,
+                      map(m.state), map(m.s6), map(m.med), map(m.vh), a, t, x);
 }
 
 template <int BI, int BJ, int M, int PREC>
-cudaError_t run_vel(const TmaMaps &m, const Vel3Args &a, const TmaTiles &t, cudaStream_t st) {
+cudaError_t run_vel(const TmaMaps &m, const Vel3Args &a, const TmaTiles &t, const VelExtra &x, cudaStream_t st) {
     constexpr int bytes = VelBoxes<BI, BJ, M, PREC>::total * 4 + 128;
     static unsigned long long devices = 0;
     cudaError_t e = smem_attr(vel3d_tma_kernel<BI, BJ, M, PREC>, bytes, devices);
     if (e != cudaSuccess) return e;
     const unsigned nblk = (unsigned)((long long)t.nkt * t.nit * t.njt * t.mgroups);
-    vel3d_tma_kernel<BI, BJ, M, PREC><<<nblk, dim3(KT, BI, 1), bytes, st>>>(map(m.own3), map(m.b3), map(m.va),
-                                                                            map(m.vb), map(m.vc), map(m.vf),
-                                                                            map(m.ve), map(m.vd), a, t);
-    return cudaGetLastError();
+    return launch_pdl(vel3d_tma_kernel<BI, BJ, M, PREC>, dim3(nblk), dim3(KT, BI, 1), bytes, st, map(m.own3), map(m.b3),
+                      map(m.va), map(m.vb), map(m.vc), map(m.vf), map(m.ve), map(m.vd), a, t, x);
 }
 
 template <int BI, int BJ, int M, int PREC = PREC_F32>
-cudaError_t stress_nm(const TmaMaps &m, const Str3Args &a, const TmaTiles &t, int nm, cudaStream_t st) {
+cudaError_t stress_nm(const TmaMaps &m, const Str3Args &a, const TmaTiles &t, const StressExtra &x, int nm,
+                      cudaStream_t st) {
     switch (nm) {
-    case 0: return run_stress<0, BI, BJ, M, PREC>(m, a, t, st);
-    case 1: return run_stress<1, BI, BJ, M, PREC>(m, a, t, st);
-    case 2: return run_stress<2, BI, BJ, M, PREC>(m, a, t, st);
-    default: return run_stress<3, BI, BJ, M, PREC>(m, a, t, st);
+    case 0: return run_stress<0, BI, BJ, M, PREC>(m, a, t, x, st);
+    case 1: return run_stress<1, BI, BJ, M, PREC>(m, a, t, x, st);
+    case 2: return run_stress<2, BI, BJ, M, PREC>(m, a, t, x, st);
+    default: return run_stress<3, BI, BJ, M, PREC>(m, a, t, x, st);
     }
 }
 
@@ -408,44 +446,44 @@ bool tma_vel_shape_ok(int bi, int bj, int mpc, int prec) {
 }
 
 cudaError_t launch_stress3d_tma(const TmaMaps &m, const Str3Args &a, const TmaTiles &t, int nm, int bi, int bj, int mpc,
-                                cudaStream_t st, int prec) {
+                                cudaStream_t st, int prec, const StressExtra &x) {
     if (prec == PREC_BF16_R)
-        return bj == 2 ? stress_nm<4, 2, 1, PREC_BF16_R>(m, a, t, nm, st) : stress_nm<4, 4, 1, PREC_BF16_R>(m, a, t, nm, st);
+        return bj == 2 ? stress_nm<4, 2, 1, PREC_BF16_R>(m, a, t, x, nm, st) : stress_nm<4, 4, 1, PREC_BF16_R>(m, a, t, x, nm, st);
     if (prec == PREC_F16_R)
-        return bj == 2 ? stress_nm<4, 2, 1, PREC_F16_R>(m, a, t, nm, st) : stress_nm<4, 4, 1, PREC_F16_R>(m, a, t, nm, st);
+        return bj == 2 ? stress_nm<4, 2, 1, PREC_F16_R>(m, a, t, x, nm, st) : stress_nm<4, 4, 1, PREC_F16_R>(m, a, t, x, nm, st);
     if (prec == PREC_F16_SR)
-        return bj == 2 ? stress_nm<4, 2, 1, PREC_F16_SR>(m, a, t, nm, st) : stress_nm<4, 4, 1, PREC_F16_SR>(m, a, t, nm, st);
+        return bj == 2 ? stress_nm<4, 2, 1, PREC_F16_SR>(m, a, t, x, nm, st) : stress_nm<4, 4, 1, PREC_F16_SR>(m, a, t, x, nm, st);
     if (mpc == 4) {
-        if (bi == 4 && bj == 1) return stress_nm<4, 1, 4>(m, a, t, nm, st);
-        return stress_nm<2, 2, 4>(m, a, t, nm, st);
+        if (bi == 4 && bj == 1) return stress_nm<4, 1, 4>(m, a, t, x, nm, st);
+        return stress_nm<2, 2, 4>(m, a, t, x, nm, st);
     }
     if (mpc == 2) {
-        if (bi == 2 && bj == 4) return stress_nm<2, 4, 2>(m, a, t, nm, st);
-        if (bi == 2 && bj == 2) return stress_nm<2, 2, 2>(m, a, t, nm, st);
-        return stress_nm<4, 2, 2>(m, a, t, nm, st);
+        if (bi == 2 && bj == 4) return stress_nm<2, 4, 2>(m, a, t, x, nm, st);
+        if (bi == 2 && bj == 2) return stress_nm<2, 2, 2>(m, a, t, x, nm, st);
+        return stress_nm<4, 2, 2>(m, a, t, x, nm, st);
     }
-    if (bi == 2 && bj == 4) return stress_nm<2, 4, 1>(m, a, t, nm, st);
-    if (bi == 4 && bj == 2) return stress_nm<4, 2, 1>(m, a, t, nm, st);
-    return stress_nm<4, 4, 1>(m, a, t, nm, st);
+    if (bi == 2 && bj == 4) return stress_nm<2, 4, 1>(m, a, t, x, nm, st);
+    if (bi == 4 && bj == 2) return stress_nm<4, 2, 1>(m, a, t, x, nm, st);
+    return stress_nm<4, 4, 1>(m, a, t, x, nm, st);
 }
 
 cudaError_t launch_vel3d_tma(const TmaMaps &m, const Vel3Args &a, const TmaTiles &t, int bi, int bj, int mpc,
-                             cudaStream_t st, int prec) {
+                             cudaStream_t st, int prec, const VelExtra &x) {
     // BF16_R keeps S in FP32: its velocity update is the FP32 one
     if (prec == PREC_F16_SR)
-        return bj == 2 ? run_vel<4, 2, 1, PREC_F16_SR>(m, a, t, st) : run_vel<4, 4, 1, PREC_F16_SR>(m, a, t, st);
+        return bj == 2 ? run_vel<4, 2, 1, PREC_F16_SR>(m, a, t, x, st) : run_vel<4, 4, 1, PREC_F16_SR>(m, a, t, x, st);
     if (mpc == 4) {
-        if (bi == 4 && bj == 1) return run_vel<4, 1, 4, PREC_F32>(m, a, t, st);
-        return run_vel<2, 2, 4, PREC_F32>(m, a, t, st);
+        if (bi == 4 && bj == 1) return run_vel<4, 1, 4, PREC_F32>(m, a, t, x, st);
+        return run_vel<2, 2, 4, PREC_F32>(m, a, t, x, st);
     }
     if (mpc == 2) {
-        if (bi == 2 && bj == 2) return run_vel<2, 2, 2, PREC_F32>(m, a, t, st);
-        if (bi == 4 && bj == 1) return run_vel<4, 1, 2, PREC_F32>(m, a, t, st);
-        return run_vel<4, 2, 2, PREC_F32>(m, a, t, st);
+        if (bi == 2 && bj == 2) return run_vel<2, 2, 2, PREC_F32>(m, a, t, x, st);
+        if (bi == 4 && bj == 1) return run_vel<4, 1, 2, PREC_F32>(m, a, t, x, st);
+        return run_vel<4, 2, 2, PREC_F32>(m, a, t, x, st);
     }
-    if (bi == 4 && bj == 4) return run_vel<4, 4, 1, PREC_F32>(m, a, t, st);
-    if (bi == 2 && bj == 2) return run_vel<2, 2, 1, PREC_F32>(m, a, t, st);
-    return run_vel<4, 2, 1, PREC_F32>(m, a, t, st);
+    if (bi == 4 && bj == 4) return run_vel<4, 4, 1, PREC_F32>(m, a, t, x, st);
+    if (bi == 2 && bj == 2) return run_vel<2, 2, 1, PREC_F32>(m, a, t, x, st);
+    return run_vel<4, 2, 1, PREC_F32>(m, a, t, x, st);
 }
 
 // ---------------------------------------------------------------------------

@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(adjt::NT, (tma::blocks_per_sm<adjt::Boxes<NM>:
     __shared__ unsigned long long limit;
     float *sm = aligned128(smraw);
     const Geo g = a.g;
-    const Tile T = tile_of<1>(t, BI, BJ);
+    const Tile T = tile_of<1>(t, BI, BJ, blockIdx.x);
     const int tx = threadIdx.x, ty = threadIdx.y, tz = threadIdx.z;
     const bool with_r = tile_has_interior(T, BI, BJ, a.ibk, a.iek, a.jbk, a.jek, a.kek);
     if (tx == 0 && ty == 0 && tz == 0) {

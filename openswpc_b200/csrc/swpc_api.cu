@@ -39,8 +39,8 @@ int cuda_check(swpc_ctx *c, cudaError_t e, const char *what) {
 int create_2d(swpc_ctx *c);
 int upload_medium_2d(swpc_ctx *c, const swpc_medium_view *m);
 int absorb_setup_2d(swpc_ctx *c, const float *gxc, const float *gxe, const float *gzc, const float *gze);
-int update_stress_2d(swpc_ctx *c, int mask);
-int update_vel_2d(swpc_ctx *c, int mask);
+int update_stress_2d(swpc_ctx *c, int mask, const Step2D &x = Step2D());
+int update_vel_2d(swpc_ctx *c, int mask, const Step2D &x = Step2D());
 int wav_store_2d(swpc_ctx *c, int it, const int *d_it);
 int vmax_2d(swpc_ctx *c, float *out);
 void destroy_2d(swpc_ctx *c);
@@ -64,10 +64,11 @@ static bool is3d(const swpc_ctx *c) { return c->kind == SWPC_KIND_3D; }
 
 static void invalidate_graph(swpc_ctx *c) {
     c->desc_dirty = true;
-    if (c->graph_exec) {
-        cudaGraphExecDestroy(c->graph_exec);
-        c->graph_exec = nullptr;
-    }
+    for (cudaGraphExec_t *g : {&c->graph_exec, &c->graph_many})
+        if (*g) {
+            cudaGraphExecDestroy(*g);
+            *g = nullptr;
+        }
 }
 namespace swpc {
 int graph_invalidate(swpc_ctx *c) {
@@ -203,7 +204,7 @@ extern "C" int swpc_create(const swpc_desc *d, swpc_ctx **out) {
         rc = create_2d(c);
     }
     if (!rc) rc = dalloc(c, &c->vmax_buf, 4);
-    if (!rc) rc = dalloc(c, &c->d_it, 1);
+    if (!rc) rc = dalloc(c, &c->d_it, 2);   // the step of graph replays, and the velocity phase's copy
     if (!rc) rc = dalloc(c, &c->d_scale, kScaleFloats);
     if (!rc) rc = dalloc(c, &c->d_exp, 24);
     if (!rc) rc = dalloc(c, &c->d_rmax, 24);
@@ -254,6 +255,10 @@ extern "C" int swpc_destroy(swpc_ctx *c) {
         if (c->gx[q]) cudaFree(c->gx[q]);
         if (c->gy[q]) cudaFree(c->gy[q]);
         if (c->gz[q]) cudaFree(c->gz[q]);
+    }
+    for (InjColumns *ic : {&c->glut_cols, &c->bf_cols, &c->green_cols}) {
+        if (ic->list) cudaFree(ic->list);
+        if (ic->col) cudaFree(ic->col);
     }
     if (c->h_vmax) cudaFreeHost(c->h_vmax);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -812,6 +817,46 @@ static int build_list(swpc_ctx *c, std::vector<InjEntry> &v, InjEntry **dptr, in
     return SWPC_OK;
 }
 
+// The same list by column, for the staged launches that add the sources of
+// the cells they update (swpc_step.cuh).  A list with ghost cells, which no
+// update reaches, with FP16 stress arrays or 2D body forces (another density
+// cell) has none and keeps its own launch.
+static int build_columns(swpc_ctx *c, const std::vector<InjEntry> &v, InjColumns &ic) {
+    if (ic.list) { cudaFree(ic.list); ic.list = nullptr; }
+    if (ic.col) { cudaFree(ic.col); ic.col = nullptr; }
+    const Geo &g = c->g;
+    std::vector<std::pair<int, int>> order;   // (column, list position): list order within a column
+    for (size_t n = 0; n < v.size(); n++) {
+        const InjEntry &e = v[n];
+        const int col = (int)(e.cell / g.Kp), k = (int)(e.cell % g.Kp) - KH + 1;
+        const int i = col % g.Ip - 2, j = is3d(c) ? col / g.Ip - 2 : 1;
+        const bool half = c->prec == SWPC_PREC_F16_SR && e.field >= SWPC_F_SXX;
+        if (k < 1 || k > g.nz || i < 1 || i > g.nx || (is3d(c) && (j < 1 || j > g.ny)) || half || e.mode > INJ_GREEN)
+            return SWPC_OK;
+        order.push_back({col, (int)n});
+    }
+    if (order.empty()) return SWPC_OK;
+    std::sort(order.begin(), order.end());
+    std::vector<InjCell> list(order.size());
+    std::vector<int> col((size_t)g.Ip * g.Jp, -1);
+    for (size_t n = 0; n < order.size(); n++) {
+        const InjEntry &e = v[order[n].second];
+        InjCell &q = list[n];
+        q.cell = e.cell;
+        q.p = (e.field < SWPC_F_SXX ? c->V[e.field - SWPC_F_VX] : c->S[e.field - SWPC_F_SXX]) + e.cell;
+        q.b = e.mode >= INJ_BF3 ? c->med[5 + e.bfield] + e.cell : nullptr;
+        q.coef = e.coef; q.src = e.src; q.mode = e.mode;
+        q.last = n + 1 == order.size() || order[n + 1].first != order[n].first;
+        if (n == 0 || order[n - 1].first != order[n].first) col[order[n].first] = (int)n;
+    }
+    RC(dalloc(c, &ic.list, list.size()));
+    RC(dalloc(c, &ic.col, col.size()));
+    CK(cudaMemcpyAsync(ic.list, list.data(), list.size() * sizeof(InjCell), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(ic.col, col.data(), col.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    return SWPC_OK;
+}
+
 static bool in_box(const swpc_ctx *c, int k, int i, int j) {
     const Geo &g = c->g;
     const int jlo = is3d(c) ? -2 : 1, jhi = is3d(c) ? g.ny + 3 : 1;
@@ -907,6 +952,7 @@ extern "C" int swpc_source_setup(swpc_ctx *c, int nsrc, const int *isrc, const i
     }
     if (bad) return set_err(c, SWPC_ERR_ARG, "source cell outside the memory box");
     RC(build_list(c, v, &c->inj_glut, &c->ninj_glut, &c->glut_serial));
+    RC(build_columns(c, v, c->glut_cols));
     c->nsrc_glut = nsrc;
     RC(stime_table(c, &c->stime_glut, nsrc, srcprm, stftype, true));
     if (c->mo_glut) { cudaFree(c->mo_glut); c->mo_glut = nullptr; }
@@ -969,6 +1015,7 @@ extern "C" int swpc_bodyforce_setup(swpc_ctx *c, int nsrc, const int *isrc, cons
     }
     if (bad) return set_err(c, SWPC_ERR_ARG, "body-force cell outside the memory box");
     RC(build_list(c, v, &c->inj_bf, &c->ninj_bf, &c->bf_serial));
+    RC(build_columns(c, v, c->bf_cols));
     c->nsrc_bf = nsrc;
     RC(stime_table(c, &c->stime_bf, nsrc, srcprm, stftype, false));
     c->dt_dxyz = c->d.dt / (c->d.dx * c->d.dy * c->d.dz);
@@ -987,6 +1034,7 @@ extern "C" int swpc_green_setup(swpc_ctx *c, int isrc, int jsrc, int ksrc, char 
         return set_err(c, SWPC_ERR_ARG, "green source cell outside the memory box");
     bool serial;
     RC(build_list(c, v, &c->inj_green, &c->ninj_green, &serial));
+    RC(build_columns(c, v, c->green_cols));
     const float prm[2] = {green_tbeg, green_trise};
     RC(stime_table(c, &c->stf_green, 1, prm, stftype, false));
     c->green_dt_dxyz = c->d.dt / (c->d.dx * c->d.dy * c->d.dz);
@@ -1117,16 +1165,28 @@ TmaTiles tma_tiles(const swpc_ctx *c, int bi, int bj, int nmem, int mpc, int nfi
     t.so = 0;
     t.ao = 0;
     t.err = c->d_err;
+    const int rest = t.njt % t.jblock;
+    t.by_nkt = FastDiv::of(t.nkt);
+    t.by_block = FastDiv::of(t.nit * t.jblock);
+    t.by_jb = FastDiv::of(t.jblock);
+    t.by_last = FastDiv::of(rest ? rest : t.jblock);
     return t;
 }
 }  // namespace swpc
 
-static int launch_stress_kernel(swpc_ctx *c, int mask);
-static int launch_vel_kernel(swpc_ctx *c, int mask);
+// What the launches of one step also do (swpc_step.cuh), for the 3D and the 2D kernels.
+struct StepExtra {
+    StressExtra str;
+    VelExtra vel;
+    Step2D d2;
+};
 
-static int launch_stress(swpc_ctx *c, int mask) {
+static int launch_stress_kernel(swpc_ctx *c, int mask, const StressExtra &x = StressExtra());
+static int launch_vel_kernel(swpc_ctx *c, int mask, const VelExtra &x = VelExtra());
+
+static int launch_stress(swpc_ctx *c, int mask, const StepExtra &x = StepExtra()) {
     RC(check_ready(c));
-    if (!is3d(c)) return update_stress_2d(c, mask);
+    if (!is3d(c)) return update_stress_2d(c, mask, x.d2);
     if (mask & 2) RC(pw_fill(c, 0));   // plane-wave side boundary before the absorber update
     if (c->abc == 1) {
         // Cerjan: the interior update over the whole domain, then the sponge
@@ -1135,10 +1195,10 @@ static int launch_stress(swpc_ctx *c, int mask) {
         if (mask & 2) RC(launch_cerjan(c, 0));
         return SWPC_OK;
     }
-    return launch_stress_kernel(c, mask);
+    return launch_stress_kernel(c, mask, x.str);
 }
 
-static int launch_stress_kernel(swpc_ctx *c, int mask) {
+static int launch_stress_kernel(swpc_ctx *c, int mask, const StressExtra &x) {
     Str3Args a;
     memset(&a, 0, sizeof(a));
     fill_geo_common(c, a.g, a.ibk, a.iek, a.jbk, a.jek, a.kek);
@@ -1162,7 +1222,7 @@ static int launch_stress_kernel(swpc_ctx *c, int mask) {
         RC(tma_ready(c));
         const TmaTiles t = tma_tiles(c, c->stress_tbi, c->stress_tbj, 1, 1, kStressFields(c), 1);
         return cuda_check(c, launch_stress3d_tma(*static_cast<TmaMaps *>(c->tmaps), a, t, c->d.nm, c->stress_tbi,
-                                                 c->stress_tbj, 1, c->stream, c->prec), "stress3d_tma launch");
+                                                 c->stress_tbj, 1, c->stream, c->prec, x), "stress3d_tma launch");
     }
     if (c->stress_march && c->prec == SWPC_PREC_F32)
         launch_stress3d_march(a, c->d.nm, c->stress_mminb, c->stress_jc, c->stream);
@@ -1170,9 +1230,9 @@ static int launch_stress_kernel(swpc_ctx *c, int mask) {
     return cuda_check(c, cudaGetLastError(), "stress3d launch");
 }
 
-static int launch_vel(swpc_ctx *c, int mask) {
+static int launch_vel(swpc_ctx *c, int mask, const StepExtra &x = StepExtra()) {
     RC(check_ready(c));
-    if (!is3d(c)) return update_vel_2d(c, mask);
+    if (!is3d(c)) return update_vel_2d(c, mask, x.d2);
     if (mask & 2) RC(pw_fill(c, 1));
     if (c->abc == 1) {
         // Cerjan (absorb__update_vel's dispatch, m_absorb.f90:60-75)
@@ -1180,10 +1240,10 @@ static int launch_vel(swpc_ctx *c, int mask) {
         if (mask & 2) RC(launch_cerjan(c, 1));
         return SWPC_OK;
     }
-    return launch_vel_kernel(c, mask);
+    return launch_vel_kernel(c, mask, x.vel);
 }
 
-static int launch_vel_kernel(swpc_ctx *c, int mask) {
+static int launch_vel_kernel(swpc_ctx *c, int mask, const VelExtra &x) {
     Vel3Args a;
     memset(&a, 0, sizeof(a));
     fill_geo_common(c, a.g, a.ibk, a.iek, a.jbk, a.jek, a.kek);
@@ -1206,7 +1266,7 @@ static int launch_vel_kernel(swpc_ctx *c, int mask) {
         RC(tma_ready(c));
         const TmaTiles t = tma_tiles(c, c->vel_tbi, c->vel_tbj, 1, 1, kVelFields, 1);
         return cuda_check(c, launch_vel3d_tma(*static_cast<TmaMaps *>(c->tmaps), a, t, c->vel_tbi, c->vel_tbj, 1,
-                                              c->stream, c->prec), "vel3d_tma launch");
+                                              c->stream, c->prec, x), "vel3d_tma launch");
     }
     if (c->prec != SWPC_PREC_F32) launch_vel3d(a, c->vel_minb, c->prec, grid, block, c->stream);
     else if (c->vel_vec) launch_vel3d_vec(a, c->vel_vminb, dim3(32, c->vel_vbi, c->vel_vbj), c->stream);
@@ -1271,9 +1331,7 @@ static int launch_green(swpc_ctx *c, int it, const int *d_it) {
     return cuda_check(c, cudaGetLastError(), "green launch");
 }
 
-static int launch_wav(swpc_ctx *c, int it, const int *d_it) {
-    if (c->nst <= 0 || c->wav_what == 0) return SWPC_OK;
-    if (!is3d(c)) return wav_store_2d(c, it, d_it);
+static Wav3Args wav_args(const swpc_ctx *c, int it, const int *d_it) {
     Wav3Args a;
     memset(&a, 0, sizeof(a));
     a.g = c->g; a.nst = c->nst; a.ntw = c->ntw; a.ntdec_w = c->ntdec_w; a.what = c->wav_what;
@@ -1286,9 +1344,20 @@ static int launch_wav(swpc_ctx *c, int it, const int *d_it) {
     memcpy(a.r40, c->r40, sizeof(a.r40)); memcpy(a.r41, c->r41, sizeof(a.r41));
     a.s_half = c->prec == SWPC_PREC_F16_SR;
     a.scale = c->d_scale;
-    // outside sampling steps the kernel only integrates u / strain
-    if (!d_it && (it - 1) % c->ntdec_w != 0 && !(c->wav_what & (SWPC_WAV_U | SWPC_WAV_STRAIN))) return SWPC_OK;
-    launch_wav3d(a, c->stream);
+    return a;
+}
+
+// whether the recorder has work at this step: outside sampling steps it only integrates u / strain
+static bool wav_due(const swpc_ctx *c, int it, const int *d_it) {
+    if (c->nst <= 0 || c->wav_what == 0) return false;
+    return d_it || (it - 1) % c->ntdec_w == 0 || (c->wav_what & (SWPC_WAV_U | SWPC_WAV_STRAIN));
+}
+
+static int launch_wav(swpc_ctx *c, int it, const int *d_it) {
+    if (c->nst <= 0 || c->wav_what == 0) return SWPC_OK;
+    if (!is3d(c)) return wav_store_2d(c, it, d_it);
+    if (!wav_due(c, it, d_it)) return SWPC_OK;
+    launch_wav3d(wav_args(c, it, d_it), c->stream);
     return cuda_check(c, cudaGetLastError(), "wav launch");
 }
 
@@ -1328,35 +1397,85 @@ extern "C" int swpc_wav_store(swpc_ctx *c, int it) { PREP(c); return launch_wav(
 // between steps) in two halves: up to global__comm_stress (half 0) and from
 // there up to global__comm_vel (half 1); with record = false the wavefield
 // advances without wav__store, green__store and snap__write
+//
+// The staged launches take the point sources, the recorder and the step
+// counter along (swpc_step.cuh) where the order of the step allows it: the
+// PML (a sponge comes between update and sources), no plane-wave mode (its
+// ghost fills come between the recorder and the update), stress traces
+// recorded on their own (the stress launch changes them).
+static bool fuses(const swpc_ctx *c) {
+    return c->stress_tma && c->vel_tma && c->slab && c->abc == 0 && !c->pw_mode;
+}
+static StepInj step_inj(const swpc_ctx *c, const InjColumns &ic, const float *stime, int nsrc, float dt_dxyz) {
+    return StepInj{ic.col, ic.list, stime, c->mo_glut, nsrc, c->d.nt, dt_dxyz};
+}
+
 static int step_half0(swpc_ctx *c, int it, const int *d_it, bool record) {
+    StepExtra x = {};
+    const bool fuse = fuses(c);
+    const bool fuse_src = fuse && c->ninj_glut > 0 && c->glut_cols.list;
+    const bool fuse_wav = fuse && record && wav_due(c, it, d_it) && !(c->wav_what & SWPC_WAV_STRESS);
+    if (fuse) {
+        const int nwav = fuse_wav ? (c->nst + kWavPerCta - 1) / kWavPerCta : 0;
+        x.str.it = x.d2.it = it;
+        x.str.d_it = x.d2.d_it = d_it;
+        x.str.nwav = x.d2.nwav = nwav;
+        if (fuse_wav) {
+            if (is3d(c)) x.str.wav = wav_args(c, it, d_it);
+            x.d2.wav = c->d_wav2d;
+            x.d2.nlist = 1;
+        }
+        if (fuse_src) {
+            x.str.inj = step_inj(c, c->glut_cols, c->stime_glut, c->nsrc_glut, c->dt_dxyz);
+            x.d2.inj = c->d_inj2d;
+        }
+        if (d_it) x.str.it_copy = c->d_it + 1;
+    }
     if (record) {
-        RC(launch_wav(c, it, d_it));
+        if (!fuse_wav) RC(launch_wav(c, it, d_it));
         RC(green_store_launch(c, it, d_it));
         RC(snap_launch(c, it, d_it));
     }
     RC(rescale_before_stress(c, it, d_it));   // FP16 forms: re-centre the scales, on the device (swpc_prec.cu)
-    RC(launch_stress(c, 3));
+    RC(launch_stress(c, 3, x));
     RC(rescale_after_stress(c));
-    return launch_glut(c, it, d_it);
+    return fuse_src ? SWPC_OK : launch_glut(c, it, d_it);
 }
-static int step_half1(swpc_ctx *c, int it, const int *d_it) {
+// *counted: the velocity launch has moved the step counter of graph replays on
+static int step_half1(swpc_ctx *c, int it, const int *d_it, bool *counted = nullptr) {
     if (c->kind == SWPC_KIND_PSV && c->ninj_bf > 0) {
         // P-SV applies body forces between the interior and absorber velocity
         // updates (src/swpc_psv/main.f90:106-110)
         RC(launch_vel(c, 1));
         RC(launch_bf(c, it, d_it));
         RC(launch_vel(c, 2));
-    } else {
-        RC(launch_vel(c, 3));
-        RC(launch_bf(c, it, d_it));
+        return launch_green(c, it, d_it);
     }
-    return launch_green(c, it, d_it);
+    StepExtra x = {};
+    const bool fuse = fuses(c), green = c->green && c->ninj_green > 0;
+    const bool fuse_bf = fuse && c->ninj_bf > 0 && c->bf_cols.list;
+    const bool fuse_green = fuse && green && c->ninj_bf <= 0 && c->green_cols.list;
+    if (fuse) {
+        x.vel.it = it;
+        x.vel.d_it = d_it ? c->d_it + 1 : nullptr;
+        if (fuse_bf) x.vel.inj = step_inj(c, c->bf_cols, c->stime_bf, c->nsrc_bf, c->dt_dxyz);
+        if (fuse_green) x.vel.inj = step_inj(c, c->green_cols, c->stf_green, 1, c->green_dt_dxyz);
+        // launches after this one would read the counter
+        const bool last = (c->ninj_bf <= 0 || fuse_bf) && (!green || fuse_green);
+        if (d_it && counted && last) {
+            x.vel.it_next = x.d2.it_next = c->d_it;
+            *counted = true;
+        }
+    }
+    RC(launch_vel(c, 3, x));
+    if (!fuse_bf) RC(launch_bf(c, it, d_it));
+    return fuse_green ? SWPC_OK : launch_green(c, it, d_it);
 }
 
-static int step_body(swpc_ctx *c, int it, const int *d_it, bool record = true) {
+static int step_body(swpc_ctx *c, int it, const int *d_it, bool record = true, bool *counted = nullptr) {
     RC(step_half0(c, it, d_it, record));
     RC(pw_comm_zero(c, 1));   // global__comm_stress (no-op outside plane-wave mode)
-    RC(step_half1(c, it, d_it));
+    RC(step_half1(c, it, d_it, counted));
     RC(pw_comm_zero(c, 0));   // global__comm_vel
     return SWPC_OK;
 }
@@ -1386,38 +1505,57 @@ int step_state(swpc_ctx *c, int it) {
 }
 }  // namespace swpc
 
-static int build_graph(swpc_ctx *c) {
-    if (c->graph_exec) return SWPC_OK;
+// `steps` steps in one graph
+static int build_graph(swpc_ctx *c, int steps, cudaGraphExec_t *exec) {
+    if (*exec) return SWPC_OK;
     RC(check_ready(c));
     PREP(c);
     cudaGraph_t graph;
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    int rc = step_body(c, 0, c->d_it);
-    if (!rc) launch_advance_it(c->d_it, c->stream);
+    int rc = SWPC_OK;
+    for (int n = 0; n < steps && !rc; n++) {
+        bool counted = false;
+        rc = step_body(c, 0, c->d_it, true, &counted);
+        if (!rc && !counted) launch_advance_it(c->d_it, c->stream);
+    }
     cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
     if (rc) return rc;
     CK(e);
-    e = cudaGraphInstantiate(&c->graph_exec, graph, 0);
+    e = cudaGraphInstantiate(exec, graph, 0);
     cudaGraphDestroy(graph);
     CK(e);
     return SWPC_OK;
 }
+
+// Steps per graph.  One graph launch costs the host about 7 us, as much as a
+// small grid's step takes on the GPU, and no launch overlaps the end of the
+// graph before it: grids whose step is short replay several steps at a time
+// (reports come every multiple of ten steps).  With ten steps against one: a
+// 40 x 36 x 32 shot 1.31 against 1.45 ms, 300 steps of a 256 x 128 P-SV model
+// 3.12 against 3.90 ms, 200 steps of a 517 x 259 SH model 1.88 against 2.32 ms.
+// A step of a million cells takes over 40 us, and the launches of one step per
+// graph are hidden behind it.
+constexpr int kGraphSteps = 10;
+constexpr long long kGraphManyCells = 1LL << 20;
 
 extern "C" int swpc_run(swpc_ctx *c, int it0, int nsteps) {
     if (!c) return SWPC_ERR_ARG;
     if (nsteps <= 0) return SWPC_OK;
     if (it0 < 1 || it0 + nsteps - 1 > c->d.nt) return set_err(c, SWPC_ERR_ARG, "time steps outside 1..nt");
     CK(cudaSetDevice(c->device));
-    RC(build_graph(c));
+    const int many = c->g.ncell <= kGraphManyCells ? nsteps / kGraphSteps : 0, rest = nsteps - many * kGraphSteps;
+    if (many) RC(build_graph(c, kGraphSteps, &c->graph_many));
+    if (rest) RC(build_graph(c, 1, &c->graph_exec));
     CK(cudaMemcpyAsync(c->d_it, &it0, sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    for (int n = 0; n < nsteps; n++) CK(cudaGraphLaunch(c->graph_exec, c->stream));
+    for (int n = 0; n < many; n++) CK(cudaGraphLaunch(c->graph_many, c->stream));
+    for (int n = 0; n < rest; n++) CK(cudaGraphLaunch(c->graph_exec, c->stream));
     return SWPC_OK;
 }
 
 extern "C" int swpc_time_steps(swpc_ctx *c, int it0, int nsteps, float *ms) {
     if (!c || !ms) return SWPC_ERR_ARG;
     CK(cudaSetDevice(c->device));
-    RC(build_graph(c));
+    RC(build_graph(c, 1, &c->graph_exec));
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));

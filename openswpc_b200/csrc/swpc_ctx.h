@@ -50,9 +50,25 @@ struct InjEntry {
     int pad;
 };
 
+// An entry of the same lists as a staged update launch applies it: the
+// entries of one column stand together in list order, the last one marked.
+struct InjCell {
+    long long cell;
+    float *p;         // the value at the cell
+    const float *b;   // the buoyancy there (body forces)
+    float coef;
+    int src, mode, last;
+};
+// One injection list by column (both null: the list has no such form).
+struct InjColumns {
+    InjCell *list = nullptr;
+    int *col = nullptr;   // per column: first entry, -1 for none
+};
+
 struct Model2D;
 struct Tile2D;
 struct Wav2Args;
+struct StepInj;
 
 }  // namespace swpc
 
@@ -122,6 +138,7 @@ struct swpc_ctx {
     int nsrc_glut = 0, nsrc_bf = 0;
     swpc::InjEntry *inj_glut = nullptr; int ninj_glut = 0; bool glut_serial = false;
     swpc::InjEntry *inj_bf = nullptr; int ninj_bf = 0; bool bf_serial = false;
+    swpc::InjColumns glut_cols, bf_cols, green_cols;   // the same lists by column
     float *stime_glut = nullptr;   // (nt, nsrc) moment rate at tbeg+(it-0.5)dt
     float *mo_glut = nullptr;      // (nsrc)
     float *stime_bf = nullptr;     // (nt, nsrc) at tbeg + it*dt
@@ -162,6 +179,7 @@ struct swpc_ctx {
     // graph
     int *d_it = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
+    cudaGraphExec_t graph_many = nullptr;   // kGraphSteps steps in one graph (small grids)
     int graph_key = -1;
 
     // 2D solvers: device model descriptor, tile list, recorder descriptor
@@ -169,6 +187,7 @@ struct swpc_ctx {
     swpc::Tile2D *d_tiles2d = nullptr;
     int ntiles2d = 0;
     swpc::Wav2Args *d_wav2d = nullptr;
+    swpc::StepInj *d_inj2d = nullptr;
     int nm2d_aux = 0;
     bool desc_dirty = true;   // device descriptors must be refreshed before the next launch
     void *maps2d = nullptr;   // tensor maps of the model (swpc::Maps2D): a kernel parameter of the staged kernels

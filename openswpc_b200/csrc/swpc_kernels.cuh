@@ -29,6 +29,17 @@ __device__ __forceinline__ float sc_iS(const float *s, int f) { return __ldg(s +
 __device__ __forceinline__ float sc_sR(const float *s, int) { return __ldg(s + 19); }
 __device__ __forceinline__ float sc_iR(const float *s, int) { return __ldg(s + 20); }
 
+// Point sources that a staged launch adds to the cells it updates
+// (swpc_step.cuh): col[column] = the column's first entry in list, -1 for none
+// (col null: no sources in this launch).
+struct StepInj {
+    const int *col;
+    const InjCell *list;
+    const float *stime, *mo;   // (nt, nsrc), (nsrc)
+    int nsrc, nt;
+    float dt_dxyz;
+};
+
 struct Vel3Args {
     Geo g;
     int ibk, iek, jbk, jek, kek;
@@ -103,6 +114,25 @@ struct Wav3Args {
     int s_half;          // S stored in FP16 (SWPC_PREC_F16_SR)
     const float *scale;
 };
+
+// What the staged stress and velocity launches of a step also do (all zero:
+// nothing).  The stress launch leaves the step in it_copy for the velocity
+// launch, which reads it there and moves the counter it_next on.
+struct StressExtra {
+    StepInj inj;
+    int nwav;            // CTAs of the recorder, before those of the tiles (kWavPerCta stations each)
+    int it;              // the step, or where graph replays keep it (d_it)
+    const int *d_it;
+    int *it_copy;
+    Wav3Args wav;
+};
+struct VelExtra {
+    StepInj inj;
+    int it;
+    const int *d_it;
+    int *it_next;
+};
+constexpr int kWavPerCta = 64;
 
 struct VmaxArgs {
     Geo g;

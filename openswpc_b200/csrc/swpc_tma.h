@@ -7,6 +7,23 @@
 
 namespace swpc {
 
+// Division of a CTA index by a launch constant as a multiply and a shift (exact
+// for 0 <= n < 2^31; m = floor(2^32 (2^s - d) / d) + 1 with 2^s the first power
+// of two >= d): the lead thread of a tile divides four times before it can
+// issue its copies.
+struct FastDiv {
+    unsigned d, m, s;
+    static FastDiv of(int n) {
+        FastDiv f{(unsigned)n, 1, 0};
+        while ((1ull << f.s) < f.d) f.s++;
+        f.m = (unsigned)(((1ull << 32) * ((1ull << f.s) - f.d)) / f.d + 1);
+        return f;
+    }
+#ifdef __CUDACC__
+    __device__ __forceinline__ int div(int n) const { return (int)((__umulhi((unsigned)n, m) + (unsigned)n) >> s); }
+#endif
+};
+
 // A staged launch: tiles of 32 (k) x bi (i) x bj (j) cells, and per tile the
 // member groups of a batch (a single run is one member).  Field coordinates
 // refer to the state slab (per member: V, S, R) and the medium slab.
@@ -23,6 +40,7 @@ struct TmaTiles {
     int f_h;             // 2-byte slab of a reduced storage form: S (F16_SR) or R (BF16_R)
     long long so, ao;    // offset between members of the state arrays and of the PML auxiliaries
     int *err;            // raised when a tile copy does not complete
+    FastDiv by_nkt, by_block, by_jb, by_last;   // nkt; nit * jblock; j tiles of a block, of the last block
 };
 
 // tiles of a staged launch over a context's grid for nmem members grouped
@@ -69,8 +87,8 @@ bool tma_encode_box(unsigned char *out, float *slab, const Geo &g, long long nf,
                     unsigned bf);
 bool tma_encode_vel(TmaMaps &m, const TmaSlabs &s, const Geo &g, int bi, int bj, int prec = 0);
 cudaError_t launch_stress3d_tma(const TmaMaps &m, const Str3Args &a, const TmaTiles &t, int nm, int bi, int bj, int mpc,
-                                cudaStream_t st, int prec = 0);
+                                cudaStream_t st, int prec = 0, const StressExtra &x = StressExtra());
 cudaError_t launch_vel3d_tma(const TmaMaps &m, const Vel3Args &a, const TmaTiles &t, int bi, int bj, int mpc,
-                             cudaStream_t st, int prec = 0);
+                             cudaStream_t st, int prec = 0, const VelExtra &x = VelExtra());
 
 }  // namespace swpc

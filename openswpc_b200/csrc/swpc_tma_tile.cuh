@@ -15,7 +15,7 @@ struct Tile {
     int k0, i0, j0, m0, nmem;   // first cell, first member, members in the group
 };
 
-// Tile and member group of this CTA: member groups fastest, then the tiles
+// Tile and member group of a CTA: member groups fastest, then the tiles
 // (the medium of a tile is re-read from L2 by the groups that follow), or with
 // t.tiles_first the tiles fastest and the groups one after another.  Within a
 // group the tiles run k fastest, then over (i, j) in blocks of t.jblock
@@ -23,14 +23,19 @@ struct Tile {
 // so that the j halo of a tile comes from tiles launched a few CTAs earlier,
 // still in L2, instead of a j plane of tiles earlier.
 template <int M>
-__device__ __forceinline__ Tile tile_of(const TmaTiles &t, int bi, int bj) {
-    const int ntile = t.nkt * t.nit * t.njt;
-    const int grp = t.tiles_first ? blockIdx.x / ntile : blockIdx.x % t.mgroups;
-    const int b = t.tiles_first ? blockIdx.x % ntile : blockIdx.x / t.mgroups;
-    const int kt = b % t.nkt, r = b / t.nkt;
-    const int jb = t.jblock, blk = r / (t.nit * jb), rem = r - blk * t.nit * jb;
-    const int nb = min(jb, t.njt - blk * jb);   // j tiles in this block (the last one may be short)
-    const int it = rem / nb, jt = blk * jb + rem % nb;
+__device__ __forceinline__ Tile tile_of(const TmaTiles &t, int bi, int bj, int cta) {
+    int grp = 0, b = cta;
+    if (t.mgroups > 1) {
+        const int ntile = t.nkt * t.nit * t.njt;
+        grp = t.tiles_first ? cta / ntile : cta % t.mgroups;
+        b = t.tiles_first ? cta % ntile : cta / t.mgroups;
+    }
+    const int r = t.by_nkt.div(b), kt = b - r * t.nkt;
+    const int blk = t.by_block.div(r), rem = r - blk * (t.nit * t.jblock);
+    const int first = blk * t.jblock;
+    const bool last = first + t.jblock > t.njt;   // the last block may be short
+    const int it = (last ? t.by_last : t.by_jb).div(rem);
+    const int jt = first + rem - it * (last ? t.njt - first : t.jblock);
     const int m0 = grp * M;
     return Tile{1 + KT * kt, 1 + bi * it, 1 + bj * jt, m0, min(M, t.nmem - m0)};
 }

@@ -1,0 +1,102 @@
+"""Point sources, recorder and step counter inside the staged launches against
+the launches of their own (flat and tile-walking kernels), bitwise."""
+import numpy as np
+import pytest
+
+from openswpc_b200 import _lib
+from openswpc_b200._lib import check
+from openswpc_b200.params import Source, Station
+from openswpc_b200.swpc2d import Batch2D, Swpc2D
+from openswpc_b200.swpc3d import Swpc3D
+from tests.models import small2d, small3d
+
+pytestmark = pytest.mark.gpu
+
+
+def _sources(p, n, seed, force):
+    """Seeded sources over the whole grid, several in the same cell and some at its edges."""
+    g = np.random.default_rng(seed)
+    out = []
+    for q in range(n):
+        if q % 3 == 2:
+            x, y, z = out[-1].x, out[-1].y, out[-1].z
+        else:
+            i = 1 if q % 7 == 3 else int(g.integers(2, p.nx))
+            j = p.ny if q % 7 == 4 else int(g.integers(2, max(p.ny, 3)))
+            k = int(g.integers(5, p.nz))
+            x, z = p.xbeg + (i - 0.5) * p.dx, p.zbeg + (k - 0.5) * p.dz
+            y = p.ybeg + (j - 0.5) * p.dy if p.ny > 1 else 0.0
+        m = g.uniform(-1, 1, 6)
+        out.append(Source(x, y, z, 0.0, 0.3, mo=1e15, mxx=m[0], myy=m[1], mzz=m[2], myz=m[3], mxz=m[4], mxy=m[5],
+                          fx=m[0] * force, fy=m[1] * force, fz=m[2] * force))
+    return out
+
+
+def _same(a, b):
+    return np.array_equal(np.ascontiguousarray(a, np.float32).view(np.uint32),
+                          np.ascontiguousarray(b, np.float32).view(np.uint32))
+
+
+# one and several steps per graph with a remainder; one and several recorder CTAs (64 stations each); grids whose
+# tiles are partial in k, i and j
+@pytest.mark.parametrize("mode", ["glut", "force", "green"])
+@pytest.mark.parametrize("dims,nsrc,nst,nt", [((21, 23, 13), 1, 1, 9), ((40, 36, 33), 40, 65, 23),
+                                              ((33, 29, 64), 7, 64, 10)])
+def test_step3d(mode, dims, nsrc, nst, nt):
+    p = small3d(nx=dims[0], ny=dims[1], nz=dims[2], na=4, nt=nt, sw_wav_u=True, sw_wav_strain=True,
+                bf_mode=mode == "force", green_mode=mode == "green", green_trise=0.5)
+    g = np.random.default_rng(5)
+    p.stations = [Station(p.xbeg + (int(g.integers(2, p.nx)) - 0.5) * p.dx,
+                          p.ybeg + (int(g.integers(2, p.ny)) - 0.5) * p.dy, 0.5, f"s{n}", "fsb") for n in range(nst)]
+    p.sources = _sources(p, nsrc, 11, 1.0)
+    runs = []
+    for flat in (False, True):
+        r = Swpc3D(p, medium_on_device=True)
+        if mode == "green":
+            r.record(what=_lib.WAV_V | _lib.WAV_U | _lib.WAV_STRAIN)
+        if flat:
+            check(r.ctx, r.lib.swpc_set_launch(r.ctx, 0, 2, 2, 1))
+            check(r.ctx, r.lib.swpc_set_launch(r.ctx, 1, 4, 2, 2))
+        r.run(1, nt)
+        runs.append([r.waveforms(w) for w in (_lib.WAV_V, _lib.WAV_U, _lib.WAV_STRAIN)] +
+                    [r.download(f) for f in range(9)])
+        r.close()
+    assert np.abs(runs[0][3]).max() > 0
+    for a, b in zip(*runs):
+        assert _same(a, b)
+
+
+@pytest.mark.parametrize("kind", ["psv", "sh"])
+@pytest.mark.parametrize("dims,nsrc,nst,nt", [((19, 14), 1, 1, 9), ((120, 61), 30, 65, 23), ((48, 33), 5, 64, 10)])
+def test_step2d(kind, dims, nsrc, nst, nt):
+    """A single run and a batch with a second model, staged and tile-walking."""
+    def params(seed):
+        p = small2d(kind, nx=dims[0] + seed, nz=dims[1], na=4, nt=nt)
+        g = np.random.default_rng(seed)
+        p.stations = [Station(p.xbeg + (int(g.integers(2, p.nx)) - 0.5) * p.dx, 0.0, 0.3, f"s{n}", "fsb")
+                      for n in range(nst)]
+        p.sources = _sources(p, nsrc, seed, 0.0)
+        return p
+
+    def out(r):
+        return [r.waveforms(w) for w in (_lib.WAV_V, _lib.WAV_U)] + [r.download(f) for f in r.field_ids.values()]
+
+    single = []
+    for flat in (False, True):
+        r = Swpc2D(params(1), kind)
+        if flat:
+            check(r.ctx, r.lib.swpc_set_launch(r.ctx, 0, 1, 1, 1))
+            check(r.ctx, r.lib.swpc_set_launch(r.ctx, 1, 1, 1, 1))
+        r.run(1, nt)
+        single.append(out(r))
+    assert max(np.abs(f).max() for f in single[0][2:]) > 0
+    for a, b in zip(*single):
+        assert _same(a, b)
+    for staged in (8, 0):
+        runs = [Swpc2D(params(s), kind) for s in (1, 2)]
+        b = Batch2D(runs)
+        b.set_staged(staged, staged)
+        b.run(1, nt)
+        for x, y in zip(out(runs[0]), single[0]):
+            assert _same(x, y)
+        b.close()
