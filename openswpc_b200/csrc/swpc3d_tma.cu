@@ -527,6 +527,18 @@ bool tma_encode_box(unsigned char *out, float *slab, const Geo &g, long long nf,
     return encode(out, slab, g, nf, bk, bi, bj, bf);
 }
 
+bool tma_encode_bytes(unsigned char *out, unsigned char *p, int Kc, int Ip, int Jp, unsigned bk, unsigned bi, unsigned bj) {
+    PFN_cuTensorMapEncodeTiled fn = encode_fn();
+    if (!fn) return false;
+    const cuuint64_t dims[4] = {(cuuint64_t)Kc, (cuuint64_t)Ip, (cuuint64_t)Jp, 1};
+    const cuuint64_t strides[3] = {(cuuint64_t)Kc, (cuuint64_t)Kc * Ip, (cuuint64_t)Kc * Ip * Jp};
+    const cuuint32_t box[4] = {bk, bi, bj, 1};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return fn(reinterpret_cast<CUtensorMap *>(out), CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, p, dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool tma_encode_stress(TmaMaps &m, const TmaSlabs &s, const Geo &g, int nm, int bi, int bj, int prec) {
     bool ok = encode(m.med, s.med, g, s.nf_med, KT, bi, bj, 7) &&
               encode(m.vh, s.state, g, s.nf_state, KB, bi + 4, bj + 4, 3);

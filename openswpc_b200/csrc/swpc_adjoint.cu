@@ -5,14 +5,18 @@
 // kernel__update_vel + absorb_p__update_vel; src/swpc_3d/m_kernel.f90:75-326,
 // src/swpc_3d/m_absorb_p.f90:126-505) is linear in the wavefield state
 // (V, S, R, PML auxiliaries).  This file applies its exact transpose, in the
-// reverse order, as two kinds of passes per half step:
-//   weights: per cell, the adjoint of that cell's own update -- memory
-//            variables and PML auxiliaries in place, and for each of the
-//            nine (field, axis) difference operators the two weights that
-//            multiply the 4th-order coefficient pair (2nd-order difference
-//            r20 and zero in absorber cells);
-//   gather:  per cell, the transposed stencil: every neighbour that read this
-//            cell adds its weight with the sign of the difference.
+// reverse order.  Each half step of the transpose has a cell-local part (the
+// adjoint of the cell's own update: memory variables and PML auxiliaries in
+// place, and one value per difference operator, its base) and a gather (the
+// transposed stencil: every neighbour that read this cell adds its base times
+// the neighbour's coefficient, with the sign of the difference).  Two kernels
+// alternate:
+//   adj_stress: gathers the velocity-phase bases U into lambda_S, then forms
+//               the stress-phase bases D from it;
+//   adj_vel:    gathers D into lambda_V, then forms the U of the step before.
+// The coefficient pair of a cell (4th order, the 2nd-order band, or absorber)
+// follows from its class, one byte a cell, so no weights are stored: an
+// interior cell's nine operators of a phase share three (U) or six (D) bases.
 // Receiver residuals enter as sources at the transposed recorder cells
 // (wav__store, src/swpc_3d/m_wav.f90:530-535).  The gradient imaging
 // condition pairs the adjoint with the forward derivatives of the same step;
@@ -30,10 +34,12 @@
 #include <algorithm>
 #include <cmath>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "swpc_ctx.h"
 #include "swpc_kernels.cuh"
+#include "swpc_step.cuh"
 #include "swpc_tma.h"
 #include "swpc_tma_ptx.cuh"
 #include "swpc_tma_tile.cuh"
@@ -51,9 +57,10 @@ struct swpc_adj_state {
     float *lV[3] = {}, *lS[6] = {}, *lR[18] = {}, *laux[18] = {};
     float *slab = nullptr;               // lV, lS, lR in the forward slab's field order (V, S, R)
     int slab_nf = 0;
-    swpc::TmaMaps *maps = nullptr;       // staged stress-phase weights: state, s6 (adjoint slab), med, vh (slots)
-    float *w40[9] = {}, *w41[9] = {};    // difference-operator weights of the stress phase
-    float *w40v[9] = {}, *w41v[9] = {};  // and of the velocity phase (formed while the stress-phase ones are read)
+    struct AdjMaps *maps = nullptr;      // tensor maps of the staged kernels
+    float *U = nullptr, *D = nullptr;    // bases of the velocity phase and of the stress phase, nine fields each
+    unsigned char *cls = nullptr;        // class of every cell of the memory box (cell_class), k pitch Kc
+    int Kc = 0;
     unsigned char *srcmask = nullptr;    // cells whose lambda_V a receiver residual changes
     int *srccells = nullptr;             // the same cells: (k, i, j) triplets, then nsrc + 1 offsets into the
                                          // contributions (station << 2 | component), in station order
@@ -73,6 +80,12 @@ struct swpc_adj_state {
     int *shell = nullptr;                // slot-box indices of the shell cells (slot box less the interior)
     int nshell = 0;
     long long bytes = 0;
+};
+
+// host copies of the tensor maps (CUtensorMap, 128 bytes, 64-byte aligned)
+struct alignas(64) AdjMaps {
+    unsigned char state[128], s6[128], med[128], v1[128], u1[128], ui[128], uj[128], uk[128], clsa[128];   // adj_stress
+    unsigned char own3[128], b3[128], da[128], db[128], dc[128], df[128], de[128], dd[128], clsb[128];     // adj_vel
 };
 
 namespace {
@@ -103,7 +116,9 @@ struct AdjVelArgs {
     float *laS[9];               // adjoint of the velocity-phase PML auxiliaries
     const float4 *gxc, *gxe, *gyc, *gye, *gzc, *gze;
     float e40[3][2], e41[3][2], r20[3], dt;
-    float *w40[9], *w41[9];
+    float *U;                    // velocity-phase bases, nine fields
+    const unsigned char *cls;
+    int Kc;
     const float *divS[3];        // forward stress divergences after the stress update (gradient, slot layout)
     float *gb[3];                // segment partials of the bx, by, bz gradient (null: none)
     SlotGeo sg;
@@ -112,7 +127,7 @@ struct AdjVelArgs {
 struct AdjStrArgs {
     Geo g;
     int ibk, iek, jbk, jek, kek, nm;
-    const float *lS[6];
+    float *lS[6];
     float *lR[18];
     const float *lam, *mu, *taup, *taus, *muyz, *muxz, *muxy;
     const int4 *band;
@@ -121,16 +136,24 @@ struct AdjStrArgs {
     const float4 *gxc, *gxe, *gyc, *gye, *gzc, *gze;
     float e40[3][2], e41[3][2], r20[3], dt;
     float c1[NM_MAX], c2[NM_MAX], d1[NM_MAX], d2;
-    float *w40[9], *w41[9];
+    const float *U;              // velocity-phase bases (gathered into lambda_S)
+    float *D;                    // stress-phase bases
+    const unsigned char *cls;
+    int Kc;
     const float *V[3];           // forward V before the stress update (gradient, slot layout)
     float *gm[5];                // segment partials of the lam, mu, muyz, muxz, muxy gradient (null: none)
     SlotGeo sg;
 };
 
-struct GatherArgs {
+// adj_vel: D gathered into lambda_V, then (next) the velocity-phase bases of the step before
+struct AdjGatherArgs {
     Geo g;
-    float *dst[6];
-    const float *w40[9], *w41[9];
+    float *lV[3];
+    const float *D;
+    float e40[3][2], e41[3][2];
+    const unsigned char *cls;
+    int Kc;
+    int ibk, iek, jbk, jek, kek;
 };
 
 __device__ __forceinline__ bool cell_of(const Geo &g, int &k, int &i, int &j) {
@@ -149,14 +172,124 @@ __device__ __forceinline__ int band_sign(const int4 bd, int k) {
     return ((p1 > p2 ? p1 : p2) >= 0) ? 1 : 0;
 }
 
-// tiles of the staged adjoint kernels: 32 x 4 x 4 cells, one thread per cell
+// Class of a cell: interior with the 4th-order pair (0) or in the 2nd-order
+// band (1), or absorber or ghost (2: its bases carry the 2nd-order factor
+// already, and are zero in ghosts).
+__global__ void cell_class_kernel(Geo g, int ibk, int iek, int jbk, int jek, int kek, const int4 *band,
+                                  unsigned char *cls, int Kc) {
+    const long long n = (long long)Kc * g.Ip * g.Jp;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
+         t += (long long)gridDim.x * blockDim.x) {
+        const long long col = t / Kc;
+        const int k = (int)(t - col * Kc) - KH + 1, i = (int)(col % g.Ip) - 2, j = (int)(col / g.Ip) - 2;
+        const bool in = i >= ibk && i <= iek && j >= jbk && j <= jek && k >= 1 && k <= kek;
+        cls[t] = in ? (unsigned char)band_sign(band[col], k) : 2;
+    }
+}
+
+// The two factors of an operator's base at a cell of class c along axis ax.
+template <class A>
+__device__ __forceinline__ float f40(const A &a, int ax, int c, float b) {
+    return c == 2 ? b : a.e40[ax][c] * b;
+}
+template <class A>
+__device__ __forceinline__ float f41(const A &a, int ax, int c, float b) {
+    return c == 2 ? 0.0f : a.e41[ax][c] * b;
+}
+
+// axis of the difference operator of velocity-phase pair p and of stress-phase pair q (x 0, y 1, z 2)
+__device__ __forceinline__ constexpr int paxis(int p) { return p % 3; }
+
+// The field that holds an interior cell's base of operator p / q: u_c of the
+// pair's velocity component, and the stress component both operators of a
+// shear pair share.
+__device__ __forceinline__ constexpr int ushare(int p) { return 4 * (p / 3); }
+__device__ __forceinline__ constexpr int dshare(int q) { return q < 3 ? q : 3 + 2 * ((q - 3) / 2); }
+
+// Transposes of the forward difference (f[e+P] - f[e]) A40 - (f[e+2P] - f[e-P]) A41
+// and of the backward one (f[e] - f[e-P]) A40 - (f[e+P] - f[e-2P]) A41, over
+// B(p, o) the base of operator p at offset o along its axis and C(ax, o) the
+// class there.
+template <class A, class B, class C>
+__device__ __forceinline__ float tfwd(const A &a, const B &base, const C &cls, int p, int ax) {
+    return f40(a, ax, cls(ax, -1), base(p, -1)) - f40(a, ax, cls(ax, 0), base(p, 0)) -
+           f41(a, ax, cls(ax, -2), base(p, -2)) + f41(a, ax, cls(ax, 1), base(p, 1));
+}
+template <class A, class B, class C>
+__device__ __forceinline__ float tbwd(const A &a, const B &base, const C &cls, int p, int ax) {
+    return f40(a, ax, cls(ax, 0), base(p, 0)) - f40(a, ax, cls(ax, 1), base(p, 1)) -
+           f41(a, ax, cls(ax, -1), base(p, -1)) + f41(a, ax, cls(ax, 2), base(p, 2));
+}
+
+// D_S^T U into the six stresses (xx yy zz yz xz xy), D_V^T D into the three velocities
+template <class A, class B, class C>
+__device__ __forceinline__ void gather_stress(const A &a, const B &U, const C &cls, float (&g)[6]) {
+    g[0] = tfwd(a, U, cls, 0, 0);
+    g[1] = tfwd(a, U, cls, 4, 1);
+    g[2] = tfwd(a, U, cls, 8, 2);
+    g[3] = tbwd(a, U, cls, 5, 2) + tbwd(a, U, cls, 7, 1);
+    g[4] = tbwd(a, U, cls, 2, 2) + tbwd(a, U, cls, 6, 0);
+    g[5] = tbwd(a, U, cls, 1, 1) + tbwd(a, U, cls, 3, 0);
+}
+template <class A, class B, class C>
+__device__ __forceinline__ void gather_vel(const A &a, const B &D, const C &cls, float (&g)[3]) {
+    g[0] = tbwd(a, D, cls, 0, 0) + tfwd(a, D, cls, 4, 1) + tfwd(a, D, cls, 6, 2);
+    g[1] = tbwd(a, D, cls, 1, 1) + tfwd(a, D, cls, 3, 0) + tfwd(a, D, cls, 8, 2);
+    g[2] = tbwd(a, D, cls, 2, 2) + tfwd(a, D, cls, 5, 0) + tfwd(a, D, cls, 7, 1);
+}
+
+// every cell of class 0
+struct Plain {
+    __device__ __forceinline__ int operator()(int, int) const { return 0; }
+};
+
+// Bases and classes from global memory (one-cell kernels): an absorber
+// neighbour has a base of its own per operator, an interior one shares.
+struct GCls {
+    const unsigned char *c;   // at the cell
+    long long PI, PJ;
+    __device__ __forceinline__ int operator()(int ax, int o) const {
+        return __ldg(c + (ax == 0 ? o * PI : ax == 1 ? o * PJ : o));
+    }
+};
+template <bool STRESS>
+struct GBase {
+    const float *b;   // at the cell, field 0
+    long long n, PI, PJ;
+    const GCls &cls;
+    __device__ __forceinline__ float operator()(int p, int o) const {
+        const int ax = STRESS ? qaxis(p) : paxis(p), sh = STRESS ? dshare(p) : ushare(p);
+        const long long f = cls(ax, o) == 2 ? p : sh;
+        return b[f * n + (ax == 0 ? o * PI : ax == 1 ? o * PJ : o)];
+    }
+};
+
+// Whether the staged tile that starts at (k0, i0, j0) reads absorber or side
+// ghost cells (then it takes nine single-axis boxes instead of the shared
+// bases with their halos), and whether an interior cell is read by such a tile
+// (it then stores its bases for all nine operators).
+template <class A>
+__device__ __forceinline__ bool tile_touches(const A &a, int k0, int i0, int j0, int bi, int bj) {
+    return i0 - 2 < a.ibk || i0 + bi + 1 > a.iek || j0 - 2 < a.jbk || j0 + bj + 1 > a.jek || k0 + tma::KT + 1 > a.kek;
+}
+template <class A>
+__device__ __forceinline__ bool read_by_touching(const A &a, int k, int i, int j, int bi, int bj) {
+    // the reading tiles lie between the ones that hold the cell shifted by -2 and by +2
+    const int il = (i - 3) / bi * bi + 1, ih = (i + 1) / bi * bi + 1;   // i >= 3 here unless the region starts at 1
+    const int jl = (j - 3) / bj * bj + 1, jh = (j + 1) / bj * bj + 1, kh = (k + 1) / tma::KT * tma::KT + 1;
+    return i < 3 || j < 3 || il - 2 < a.ibk || ih + bi + 1 > a.iek || jl - 2 < a.jbk || jh + bj + 1 > a.jek ||
+           kh + tma::KT + 1 > a.kek;
+}
+
+// tiles of the staged adjoint kernels: adj_stress 32 x 4 x 2 cells, one thread
+// per cell; adj_vel 32 x 4 x 4 cells, one thread per (k, i)
 namespace adjt {
 using namespace tma;
-constexpr int BI = 4, BJ = 4, NT = KT * BI * BJ;
+constexpr int BI = 4, BJA = 2, BJB = 4, NT = KT * BI * BJA;
 }  // namespace adjt
 
 // ---------------------------------------------------------------------------
-// transpose of the velocity update: weights
+// transpose of the velocity update: bases
 // pairs p: 0 (Vx,Sxx,x) 1 (Vx,Sxy,y) 2 (Vx,Sxz,z) 3 (Vy,Sxy,x) 4 (Vy,Syy,y)
 //          5 (Vy,Syz,z) 6 (Vz,Sxz,x) 7 (Vz,Syz,y) 8 (Vz,Szz,z)
 // ---------------------------------------------------------------------------
@@ -188,57 +321,73 @@ __device__ __forceinline__ void stress_divergence(const float (&e40)[3][2], cons
          + (S(2, 1, 0, 0) - S(2, 0, 0, 0)) * re40z - (S(2, 2, 0, 0) - S(2, -1, 0, 0)) * re41z;
 }
 
-struct Gb3 {
-    float v[3];
+// What a cell's local part reads besides its operands, loaded early: an
+// interior cell's imaging sums (and in the velocity phase its forward stress
+// divergences, v[3..5]), or an absorber cell's nine adjoint auxiliaries with
+// their place in the compact arrays.
+struct AdjPre {
+    float v[9];
+    int q;
 };
-__device__ __forceinline__ Gb3 gb_load(const AdjVelArgs &a, long long e) {
-    Gb3 g;
+__device__ __forceinline__ void aux_pre(AdjPre &x, float *const *aux, const int2 *pmlcol, long long col, int k) {
+    const int2 pc = __ldg(&pmlcol[col]);
+    x.q = pc.y + (k - pc.x);
 #pragma unroll
-    for (int q = 0; q < 3; q++) g.v[q] = a.gb[q][e];
-    return g;
+    for (int n = 0; n < 9; n++) x.v[n] = aux[n][x.q];
+}
+__device__ __forceinline__ AdjPre vel_pre(const AdjVelArgs &a, bool interior, long long col, int k, int i, int j,
+                                          long long e) {
+    AdjPre x = {};
+    if (!interior) {
+        aux_pre(x, a.laS, a.pmlcol, col, k);
+    } else if (a.gb[0]) {
+        const long long es = slot_index(a.sg, k, i, j);
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            x.v[q] = a.gb[q][e];
+            x.v[3 + q] = __ldcs(a.divS[q] + es);
+        }
+    }
+    return x;
 }
 
-// interior (s >= 0: band sign) or absorber (s < 0) cell
+// interior or absorber cell
 template <class O>
-__device__ __forceinline__ void adj_vel_cell(const AdjVelArgs &a, const O &o, long long col, int k, int i, int j,
-                                             long long e, int s, const Gb3 &g0) {
+__device__ __forceinline__ void adj_vel_cell(const AdjVelArgs &a, const O &o, int k, int i, int j, long long e,
+                                             bool interior, const AdjPre &x) {
     const float dt = a.dt;
     const float l[3] = {o.lV(0), o.lV(1), o.lV(2)};
     const float u[3] = {o.b(0) * dt * l[0], o.b(1) * dt * l[1], o.b(2) * dt * l[2]};
-    if (s >= 0) {
+    if (interior) {
 #pragma unroll
-        for (int p = 0; p < 9; p++) {
-            const int c = p / 3, ax = p % 3;
-            a.w40[p][e] = a.e40[ax][s] * u[c];
-            a.w41[p][e] = a.e41[ax][s] * u[c];
-        }
+        for (int c = 0; c < 3; c++) a.U[ushare(3 * c) * a.g.ncell + e] = u[c];
+        if (read_by_touching(a, k, i, j, adjt::BI, adjt::BJA))
+#pragma unroll
+            for (int p = 0; p < 9; p++)
+                if (p != ushare(p)) a.U[p * a.g.ncell + e] = u[p / 3];
         if (a.gb[0]) {
             // d(Vx)/d(bx) = d3Sx3 * dt, the divergences of the forward S after
             // the stress update (formed once per step of the recompute)
 #pragma unroll
-            const long long es = slot_index(a.sg, k, i, j);
-            for (int q = 0; q < 3; q++) a.gb[q][e] = (float)(g0.v[q] + (double)l[q] * __ldcs(a.divS[q] + es) * dt);
+            for (int q = 0; q < 3; q++) a.gb[q][e] = (float)(x.v[q] + (double)l[q] * x.v[3 + q] * dt);
         }
         return;
     }
     // absorber cell: V += b * (g.x * D + g.y * aux_old) * dt, aux = g.z * aux + g.w * D * dt
-    const int2 pc = __ldg(&a.pmlcol[col]);
-    const long long q = (long long)pc.y + (k - pc.x);
     const float4 gp[9] = {__ldg(&a.gxe[i - 1]), __ldg(&a.gyc[j - 1]), __ldg(&a.gzc[k - 1]),
                           __ldg(&a.gxc[i - 1]), __ldg(&a.gye[j - 1]), __ldg(&a.gzc[k - 1]),
                           __ldg(&a.gxc[i - 1]), __ldg(&a.gyc[j - 1]), __ldg(&a.gze[k - 1])};
 #pragma unroll
     for (int p = 0; p < 9; p++) {
         const int c = p / 3, ax = p % 3;
-        const float la = a.laS[p][q];
+        const float la = x.v[p];
         const float lD = u[c] * gp[p].x + gp[p].w * dt * la;
-        a.laS[p][q] = gp[p].z * la + u[c] * gp[p].y;
-        a.w40[p][e] = a.r20[ax] * lD;
-        a.w41[p][e] = 0.0f;
+        a.laS[p][x.q] = gp[p].z * la + u[c] * gp[p].y;
+        a.U[p * a.g.ncell + e] = a.r20[ax] * lD;
     }
 }
 
-__global__ void __launch_bounds__(128) adj_vel_weights_kernel(const AdjVelArgs a) {
+__global__ void __launch_bounds__(128) adj_vel_bases_kernel(const AdjVelArgs a) {
     const Geo g = a.g;
     int k, i, j;
     if (!cell_of(g, k, i, j)) return;
@@ -246,9 +395,7 @@ __global__ void __launch_bounds__(128) adj_vel_weights_kernel(const AdjVelArgs a
     const long long e = col * g.Kp + (k - 1 + KH);
     const GAdjVelOps o{a, e};
     const bool interior = i >= a.ibk && i <= a.iek && j >= a.jbk && j <= a.jek && k <= a.kek;
-    const int s = interior ? band_sign(__ldg(&a.band[col]), k) : -1;
-    const Gb3 g0 = (interior && a.gb[0]) ? gb_load(a, e) : Gb3{};
-    adj_vel_cell(a, o, col, k, i, j, e, s, g0);
+    adj_vel_cell(a, o, k, i, j, e, interior, vel_pre(a, interior, col, k, i, j, e));
 }
 
 __global__ void mark_cells_kernel(Geo g, const int *cells, int n, unsigned char *mask) {
@@ -256,32 +403,8 @@ __global__ void mark_cells_kernel(Geo g, const int *cells, int n, unsigned char 
     if (q < n) mask[cell_index(g, cells[3 * q], cells[3 * q + 1], cells[3 * q + 2])] = 1;
 }
 
-// transpose of a forward difference (f[e+P] - f[e]) * A40 - (f[e+2P] - f[e-P]) * A41
-__device__ __forceinline__ float tfwd(const float *w40, const float *w41, long long f, long long P) {
-    return w40[f - P] - w40[f] - w41[f - 2 * P] + w41[f + P];
-}
-// transpose of a backward difference (f[e] - f[e-P]) * A40 - (f[e+P] - f[e-2P]) * A41
-__device__ __forceinline__ float tbwd(const float *w40, const float *w41, long long f, long long P) {
-    return w40[f] - w40[f + P] - w41[f - P] + w41[f + 2 * P];
-}
-
-// lambda_S += D_S^T weights (dst = lS: xx yy zz yz xz xy)
-__global__ void __launch_bounds__(128) adj_vel_gather_kernel(const GatherArgs a) {
-    const Geo g = a.g;
-    int k, i, j;
-    if (!cell_of(g, k, i, j)) return;
-    const long long f = cell_index(g, k, i, j);
-    const long long PI = g.Kp, PJ = (long long)g.Kp * g.Ip;
-    a.dst[0][f] += tfwd(a.w40[0], a.w41[0], f, PI);
-    a.dst[1][f] += tfwd(a.w40[4], a.w41[4], f, PJ);
-    a.dst[2][f] += tfwd(a.w40[8], a.w41[8], f, 1);
-    a.dst[3][f] += tbwd(a.w40[5], a.w41[5], f, 1) + tbwd(a.w40[7], a.w41[7], f, PJ);
-    a.dst[4][f] += tbwd(a.w40[2], a.w41[2], f, 1) + tbwd(a.w40[6], a.w41[6], f, PI);
-    a.dst[5][f] += tbwd(a.w40[1], a.w41[1], f, PJ) + tbwd(a.w40[3], a.w41[3], f, PI);
-}
-
 // ---------------------------------------------------------------------------
-// transpose of the stress update: weights
+// transpose of the stress update
 // pairs q: 0 (Vx,x,bwd) 1 (Vy,y,bwd) 2 (Vz,z,bwd) 3 (Vy,x,fwd) 4 (Vx,y,fwd)
 //          5 (Vz,x,fwd) 6 (Vx,z,fwd) 7 (Vz,y,fwd) 8 (Vy,z,fwd)
 // ---------------------------------------------------------------------------
@@ -293,7 +416,8 @@ __global__ void __launch_bounds__(128) adj_vel_gather_kernel(const GatherArgs a)
 struct GAdjStrOps {
     const AdjStrArgs &a;
     long long e, es, PI, PJ;     // es, PI, PJ: V in the slot layout
-    __device__ __forceinline__ float lS(int c) const { return a.lS[c][e]; }
+    float l[6];                  // lambda_S with the gathered part
+    __device__ __forceinline__ float lS(int c) const { return l[c]; }
     __device__ __forceinline__ float lR(int q) const { return a.lR[q][e]; }
     __device__ __forceinline__ float med(int m) const {
         const float *p = m == 0 ? a.mu : m == 1 ? a.lam : m == 2 ? a.taup : m == 3 ? a.taus
@@ -305,21 +429,21 @@ struct GAdjStrOps {
     }
 };
 
-// the five imaging accumulators of a cell before this step (read early by
-// the staged kernel)
-struct Gm5 {
-    float v[5];
-};
-__device__ __forceinline__ Gm5 gm_load(const AdjStrArgs &a, long long e) {
-    Gm5 g;
+__device__ __forceinline__ AdjPre stress_pre(const AdjStrArgs &a, bool interior, long long col, int k, long long e) {
+    AdjPre x = {};
+    if (!interior) {
+        aux_pre(x, a.laV, a.pmlcol, col, k);
+    } else if (a.gm[0]) {
 #pragma unroll
-    for (int q = 0; q < 5; q++) g.v[q] = a.gm[q][e];
-    return g;
+        for (int q = 0; q < 5; q++) x.v[q] = a.gm[q][e];
+    }
+    return x;
 }
 
 // interior cell (s: band sign)
 template <int NM, class O>
-__device__ __forceinline__ void adj_stress_interior(const AdjStrArgs &a, const O &o, int s, long long e, const Gm5 &g0) {
+__device__ __forceinline__ void adj_stress_interior(const AdjStrArgs &a, const O &o, int s, int k, int i, int j,
+                                                    long long e, const AdjPre &g0) {
     const float dt = a.dt;
     float al[6];
 #pragma unroll
@@ -359,11 +483,10 @@ __device__ __forceinline__ void adj_stress_interior(const AdjStrArgs &a, const O
     const float lxz = muc[1] * taus_plus1 * al[4] + muc[1] * taus1 * lF[4];
     const float lxy = muc[2] * taus_plus1 * al[5] + muc[2] * taus1 * lF[5];
     ld[3] = lxy; ld[4] = lxy; ld[5] = lxz; ld[6] = lxz; ld[7] = lyz; ld[8] = lyz;
+    const bool all = read_by_touching(a, k, i, j, adjt::BI, adjt::BJB);
 #pragma unroll
-    for (int q = 0; q < 9; q++) {
-        a.w40[q][e] = a.e40[qaxis(q)][s] * ld[q];
-        a.w41[q][e] = a.e41[qaxis(q)][s] * ld[q];
-    }
+    for (int q = 0; q < 9; q++)
+        if (q == dshare(q) || all) a.D[q * a.g.ncell + e] = ld[q];
     if (a.gm[0]) {
         // forward strain rates on V before the stress update
         const float re40x = a.e40[0][s], re41x = a.e41[0][s], re40y = a.e40[1][s], re41y = a.e41[1][s];
@@ -397,15 +520,13 @@ __device__ __forceinline__ void adj_stress_interior(const AdjStrArgs &a, const O
 
 // absorber cell (m_absorb_p.f90:445-491)
 template <class O>
-__device__ __forceinline__ void adj_stress_absorber(const AdjStrArgs &a, const O &o, long long col, int k, int i,
-                                                    int j, long long e) {
+__device__ __forceinline__ void adj_stress_absorber(const AdjStrArgs &a, const O &o, int k, int i, int j, long long e,
+                                                    const AdjPre &x) {
     const float dt = a.dt;
     float al[6];
 #pragma unroll
     for (int c = 0; c < 6; c++) al[c] = o.lS(c) * dt;
     const float mu = o.med(0), lam = o.med(1);
-    const int2 pc = __ldg(&a.pmlcol[col]);
-    const long long q = (long long)pc.y + (k - pc.x);
     const float4 gxc = __ldg(&a.gxc[i - 1]), gxe = __ldg(&a.gxe[i - 1]);
     const float4 gyc = __ldg(&a.gyc[j - 1]), gye = __ldg(&a.gye[j - 1]);
     const float4 gzc = __ldg(&a.gzc[k - 1]), gze = __ldg(&a.gze[k - 1]);
@@ -420,9 +541,9 @@ __device__ __forceinline__ void adj_stress_absorber(const AdjStrArgs &a, const O
         const int ia[3] = {0, 4, 8};
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-            const float la = a.laV[ia[c]][q];
+            const float la = x.v[ia[c]];
             ld[c] = gg[c].x * lA[c] + gg[c].w * dt * la;
-            a.laV[ia[c]][q] = gg[c].z * la + gg[c].y * lA[c];
+            a.laV[ia[c]][x.q] = gg[c].z * la + gg[c].y * lA[c];
         }
     }
     // shear: S' = S + mu_c (g1.x D1 + g2.x D2 + g1.y aux1 + g2.y aux2) dt
@@ -437,90 +558,162 @@ __device__ __forceinline__ void adj_stress_absorber(const AdjStrArgs &a, const O
         const float bb[6] = {bxy, bxy, bxz, bxz, byz, byz};
 #pragma unroll
         for (int n = 0; n < 6; n++) {
-            const float la = a.laV[ia[n]][q];
+            const float la = x.v[ia[n]];
             ld[3 + n] = gg[n].x * bb[n] + gg[n].w * dt * la;
-            a.laV[ia[n]][q] = gg[n].z * la + gg[n].y * bb[n];
+            a.laV[ia[n]][x.q] = gg[n].z * la + gg[n].y * bb[n];
         }
     }
 #pragma unroll
-    for (int qq = 0; qq < 9; qq++) {
-        a.w40[qq][e] = a.r20[qaxis(qq)] * ld[qq];
-        a.w41[qq][e] = 0.0f;
-    }
+    for (int qq = 0; qq < 9; qq++) a.D[qq * a.g.ncell + e] = a.r20[qaxis(qq)] * ld[qq];
 }
 
 template <int NM>
-__global__ void __launch_bounds__(128) adj_stress_weights_kernel(const AdjStrArgs a) {
+__global__ void __launch_bounds__(128) adj_stress_kernel(const AdjStrArgs a) {
     const Geo g = a.g;
     int k, i, j;
     if (!cell_of(g, k, i, j)) return;
     const long long col = col_index(g, i, j);
     const long long e = col * g.Kp + (k - 1 + KH);
-    const GAdjStrOps o{a, e, slot_index(a.sg, k, i, j), (long long)a.sg.Kp, (long long)a.sg.Kp * a.sg.Ip};
-    if (i >= a.ibk && i <= a.iek && j >= a.jbk && j <= a.jek && k <= a.kek) {
-        const Gm5 g0 = a.gm[0] ? gm_load(a, e) : Gm5{};
-        adj_stress_interior<NM>(a, o, band_sign(__ldg(&a.band[col]), k), e, g0);
-    } else {
-        adj_stress_absorber(a, o, col, k, i, j, e);
+    const GCls cls{a.cls + col * a.Kc + (k - 1 + KH), a.Kc, (long long)a.Kc * g.Ip};
+    const GBase<false> U{a.U + e, g.ncell, g.Kp, (long long)g.Kp * g.Ip, cls};
+    float gs[6];
+    gather_stress(a, U, cls, gs);
+    GAdjStrOps o{a, e, slot_index(a.sg, k, i, j), (long long)a.sg.Kp, (long long)a.sg.Kp * a.sg.Ip, {}};
+#pragma unroll
+    for (int c = 0; c < 6; c++) {
+        o.l[c] = a.lS[c][e] + gs[c];
+        a.lS[c][e] = o.l[c];
     }
+    const int s = cls(0, 0);
+    const AdjPre x = stress_pre(a, s < 2, col, k, e);
+    if (s < 2) adj_stress_interior<NM>(a, o, s, k, i, j, e, x);
+    else adj_stress_absorber(a, o, k, i, j, e, x);
 }
 
-// The staged form (see swpc3d_tma.cu for the design): a CTA per tile of
-// 32 x 4 x 4 cells whose medium (the context's slab), adjoint S and R (the
-// adjoint slab, S alone in tiles without interior cells) and, for the
-// gradient, the forward V with its halo (one slot of the recompute) arrive
-// by bulk tensor copies; the imaging accumulators and band signs are read
-// while the copies travel.
+// The staged form (see swpc3d_tma.cu for the design): the medium of a tile of
+// 32 x 4 x 2 cells (the context's slab), its adjoint S and R (the adjoint
+// slab, S alone in tiles without interior cells), the bases U with their
+// halos, the cell classes and, for the gradient, the forward V with its halo
+// (one slot of the recompute) arrive by bulk tensor copies; the imaging
+// accumulators are read while the copies travel.  The tile takes 68 KB, so
+// three CTAs fit an SM (a 32 x 4 x 4 tile takes 116 KB: one).
 namespace adjt {
 template <int NM>
 struct Boxes {
-    static constexpr int n = NT;
-    static constexpr int nMed = 7 * n, nState = (6 + 6 * NM) * n, nV = 3 * (BJ + 4) * (BI + 4) * KB;
-    static constexpr int oState = up32(nMed), oV = oState + up32(nState), total = oV + up32(nV);
-    __host__ __device__ static constexpr unsigned bytes(bool with_r, bool grad) {
-        return 4u * (unsigned)(nMed + (with_r ? nState : 6 * n) + (grad ? nV : 0));
+    static constexpr int BJ = BJA, n = NT;
+    static constexpr int nMed = 7 * n, nState = (6 + 6 * NM) * n;
+    // one component with the halo of its three differences; one operator's halo in i, j or k
+    static constexpr int n1 = up32((BJ + 3) * (BI + 3) * KB);
+    static constexpr int nI = BJ * (BI + 3) * KT, nJ = (BJ + 3) * BI * KT, nK = BJ * BI * KB;
+    static constexpr int nU = 3 * n1 > 3 * (nI + nJ + nK) ? 3 * n1 : 3 * (nI + nJ + nK);
+    static constexpr int KC = KT + 16, nCls = (BJ + 4) * (BI + 4) * KC;   // bytes
+    static constexpr int oState = up32(nMed), oU = oState + up32(nState), oV = oU + up32(nU), oC = oV + 3 * n1,
+                         total = oC + up32(nCls / 4);
+    __host__ __device__ static constexpr unsigned bytes(bool with_r, bool grad, bool touch) {
+        return 4u * (unsigned)(nMed + (with_r ? nState : 6 * n) + (grad ? 3 * (BJ + 3) * (BI + 3) * KB : 0) +
+                               (touch ? 3 * (nI + nJ + nK) : 3 * (BJ + 3) * (BI + 3) * KB)) + (unsigned)nCls;
     }
 };
 template <int NM>
 struct SOps {
     const float *sm;
     int tx, ty, tz;
+    float l[6];
     using L = Boxes<NM>;
-    __device__ __forceinline__ int at(int f) const { return ((f * BJ + tz) * BI + ty) * KT + tx; }
-    __device__ __forceinline__ float lS(int c) const { return sm[L::oState + at(c)]; }
+    __device__ __forceinline__ int at(int f) const { return ((f * BJA + tz) * BI + ty) * KT + tx; }
+    __device__ __forceinline__ float lS(int c) const { return l[c]; }
     __device__ __forceinline__ float lR(int q) const { return sm[L::oState + at(6 + (q / 3) * NM + q % 3)]; }
     // medium box: lam mu taup taus muyz muxz muxy
     __device__ __forceinline__ float med(int m) const { return sm[at(m == 0 ? 1 : m == 1 ? 0 : m)]; }
-    __device__ __forceinline__ float V(int c, int dk, int di, int dj) const {
-        return sm[L::oV + ((c * (BJ + 4) + tz + 2 + dj) * (BI + 4) + ty + 2 + di) * KB + tx + 4 + dk];
+    // a component's box starts at i0-2, j0-1 (x), i0-1, j0-2 (y), i0-1, j0-1 (z), k0-4
+    __device__ __forceinline__ int comp(int c, int dk, int di, int dj) const {
+        return c * L::n1 + ((tz + dj + (c == 1 ? 2 : 1)) * (BI + 3) + ty + di + (c == 0 ? 2 : 1)) * KB + tx + 4 + dk;
+    }
+    __device__ __forceinline__ float V(int c, int dk, int di, int dj) const { return sm[L::oV + comp(c, dk, di, dj)]; }
+};
+// classes of the tile with its halo: box from (k0-8, i0-2, j0-2)
+template <int KC>
+struct SCls {
+    const unsigned char *c;   // at the cell
+    __device__ __forceinline__ int operator()(int ax, int o) const {
+        return c[ax == 0 ? o * KC : ax == 1 ? o * KC * (BI + 4) : o];
     }
 };
+// U of tiles inside the region: the shared bases as components with halos
+template <int NM>
+struct UShared {
+    const SOps<NM> &o;
+    __device__ __forceinline__ float operator()(int p, int d) const {
+        const int ax = paxis(p);
+        return o.sm[Boxes<NM>::oU + o.comp(p / 3, ax == 2 ? d : 0, ax == 0 ? d : 0, ax == 1 ? d : 0)];
+    }
+};
+// U of the others: nine operators, each with the halo of its axis (field p / 3 of its axis's three)
+template <int NM>
+struct UOwn {
+    const SOps<NM> &o;
+    using L = Boxes<NM>;
+    __device__ __forceinline__ float operator()(int p, int d) const {
+        const int c = p / 3, lo = p == 0 || p == 4 || p == 8 ? 2 : 1;   // first halo cell of a forward / backward transpose
+        if (paxis(p) == 0) return o.sm[L::oU + c * L::nI + (o.tz * (BI + 3) + o.ty + lo + d) * KT + o.tx];
+        if (paxis(p) == 1) return o.sm[L::oU + 3 * L::nI + c * L::nJ + ((o.tz + lo + d) * BI + o.ty) * KT + o.tx];
+        return o.sm[L::oU + 3 * (L::nI + L::nJ) + c * L::nK + (o.tz * BI + o.ty) * KB + o.tx + 4 + d];
+    }
+};
+
+// whether any of the n bytes (a multiple of 4) at p is set, over the CTA
+__device__ __forceinline__ bool any_byte(const unsigned char *p, int n, int t, int nthreads) {
+    unsigned v = 0;
+    for (int q = t; q < n / 4; q += nthreads) v |= reinterpret_cast<const unsigned *>(p)[q];
+    return __syncthreads_or(v != 0);
+}
 }  // namespace adjt
+
+struct StrMaps {
+    CUtensorMap state, s6, med, v1, u1, ui, uj, uk, cls;
+};
 
 template <int NM, bool GRAD>
 __global__ void __launch_bounds__(adjt::NT, (tma::blocks_per_sm<adjt::Boxes<NM>::total, adjt::NT>()))
-    adj_stress_tma_kernel(const __grid_constant__ CUtensorMap tm_state, const __grid_constant__ CUtensorMap tm_s,
-                          const __grid_constant__ CUtensorMap tm_med, const __grid_constant__ CUtensorMap tm_v,
-                          const AdjStrArgs a, const TmaTiles t, int fv) {
+    adj_stress_tma_kernel(const __grid_constant__ StrMaps tm, const __grid_constant__ AdjStrArgs a,
+                          const __grid_constant__ TmaTiles t, int fv) {
     using namespace adjt;
     using L = Boxes<NM>;
+    constexpr int BJ = BJA;
     extern __shared__ __align__(128) unsigned char smraw[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ unsigned long long limit;
     float *sm = aligned128(smraw);
-    const Geo g = a.g;
+    const Geo &g = a.g;
     const Tile T = tile_of<1>(t, BI, BJ, blockIdx.x);
     const int tx = threadIdx.x, ty = threadIdx.y, tz = threadIdx.z;
     const bool with_r = tile_has_interior(T, BI, BJ, a.ibk, a.iek, a.jbk, a.jek, a.kek);
+    const bool touch = tile_touches(a, T.k0, T.i0, T.j0, BI, BJ);
     if (tx == 0 && ty == 0 && tz == 0) {
         // the copies go out first; the error word is read while they travel
-        stage_init(&bar, L::bytes(with_r, GRAD));
-        const int x0 = T.k0 - 1 + KH;
-        load_4d(sm, &tm_med, x0, T.i0 + 2, T.j0 + 2, t.f_med, &bar);
-        load_4d(sm + L::oState, with_r ? &tm_state : &tm_s, x0, T.i0 + 2, T.j0 + 2, t.f_state, &bar);
-        // V with its halo from the slot: the box starts at cell (k0 - 4, i0 - 2, j0 - 2); tiles of the absorber
-        // may reach outside the slot box, where the copy fills zeros that no interior cell reads
-        if (GRAD) load_4d(sm + L::oV, &tm_v, x0 - 4, T.i0 - 2 - a.sg.i0, T.j0 - 2 - a.sg.j0, fv, &bar);
+        stage_init(&bar, L::bytes(with_r, GRAD, touch));
+        pdl_wait();
+        const int x0 = T.k0 - 1 + KH, ic = T.i0 + 2, jc = T.j0 + 2;
+        load_4d(sm, &tm.med, x0, ic, jc, t.f_med, &bar);
+        load_4d(sm + L::oState, with_r ? &tm.state : &tm.s6, x0, ic, jc, t.f_state, &bar);
+        float *u = sm + L::oU;
+        if (!touch) {
+            for (int c = 0; c < 3; c++)
+                load_4d(u + c * L::n1, &tm.u1, x0 - 4, ic - (c == 0 ? 2 : 1), jc - (c == 1 ? 2 : 1), ushare(3 * c), &bar);
+        } else {
+            for (int c = 0; c < 3; c++) {
+                load_4d(u + c * L::nI, &tm.ui, x0, ic - (c == 0 ? 2 : 1), jc, 3 * c, &bar);
+                load_4d(u + 3 * L::nI + c * L::nJ, &tm.uj, x0, ic, jc - (c == 1 ? 2 : 1), 3 * c + 1, &bar);
+                load_4d(u + 3 * (L::nI + L::nJ) + c * L::nK, &tm.uk, x0 - 4, ic, jc, 3 * c + 2, &bar);
+            }
+        }
+        // V with its halo from the slot; tiles of the absorber may reach outside the slot box, where the copy fills
+        // zeros that no interior cell reads
+        if (GRAD)
+            for (int c = 0; c < 3; c++)
+                load_4d(sm + L::oV + c * L::n1, &tm.v1, x0 - 4, T.i0 - a.sg.i0 - (c == 0 ? 2 : 1),
+                        T.j0 - a.sg.j0 - (c == 1 ? 2 : 1), fv + c, &bar);
+        load_4d(sm + L::oC, &tm.cls, x0 - 8, ic - 2, jc - 2, 0, &bar);
         limit = wait_limit(t.err);
     }
     const int k = T.k0 + tx, i = T.i0 + ty, j = T.j0 + tz;
@@ -528,28 +721,32 @@ __global__ void __launch_bounds__(adjt::NT, (tma::blocks_per_sm<adjt::Boxes<NM>:
     const bool interior = i >= a.ibk && i <= a.iek && j >= a.jbk && j <= a.jek && k <= a.kek;
     const long long col = col_index(g, i, j);
     const long long e = col * g.Kp + (k - 1 + KH);
-    const int sgn = (mine && interior) ? band_sign(__ldg(&a.band[col]), k) : 0;
-    const Gm5 g0 = (GRAD && mine && interior) ? gm_load(a, e) : Gm5{};
+    pdl_wait();
+    pdl_launch();
+    const AdjPre x = mine ? stress_pre(a, interior, col, k, e) : AdjPre{};
     __syncthreads();   // barrier initialised, wait limit set
-    if (!wait_tiles(&bar, t.err, limit) || !mine) return;   // the copy failed, or no cell here
-    const SOps<NM> o{sm, tx, ty, tz};
-    if (interior) adj_stress_interior<NM>(a, o, sgn, e, g0);
-    else adj_stress_absorber(a, o, col, k, i, j, e);
+    const bool ok = wait_tiles(&bar, t.err, limit);
+    const unsigned char *cb = reinterpret_cast<const unsigned char *>(sm + L::oC);
+    const int tid = (tz * BI + ty) * KT + tx;
+    const bool plain = !any_byte(cb, L::nCls, tid, NT);   // 4th order throughout (implies that no absorber is near)
+    if (!ok || !mine) return;   // the copy failed, or no cell here
+    SOps<NM> o{sm, tx, ty, tz, {}};
+    const SCls<L::KC> cls{cb + ((tz + 2) * (BI + 4) + ty + 2) * L::KC + tx + 8};
+    float gs[6];
+    if (touch) gather_stress(a, UOwn<NM>{o}, cls, gs);
+    else if (plain) gather_stress(a, UShared<NM>{o}, Plain{}, gs);
+    else gather_stress(a, UShared<NM>{o}, cls, gs);
+#pragma unroll
+    for (int c = 0; c < 6; c++) {
+        o.l[c] = sm[L::oState + o.at(c)] + gs[c];
+        a.lS[c][e] = o.l[c];
+    }
+    if (interior) adj_stress_interior<NM>(a, o, plain ? 0 : cls(0, 0), k, i, j, e, x);
+    else adj_stress_absorber(a, o, k, i, j, e, x);
 }
 
-// lambda_V += D_V^T weights (dst = lV: x y z)
-__global__ void __launch_bounds__(128) adj_stress_gather_kernel(const GatherArgs a) {
-    const Geo g = a.g;
-    int k, i, j;
-    if (!cell_of(g, k, i, j)) return;
-    const long long f = cell_index(g, k, i, j);
-    const long long PI = g.Kp, PJ = (long long)g.Kp * g.Ip;
-    a.dst[0][f] += tbwd(a.w40[0], a.w41[0], f, PI) + tfwd(a.w40[4], a.w41[4], f, PJ) + tfwd(a.w40[6], a.w41[6], f, 1);
-    a.dst[1][f] += tbwd(a.w40[1], a.w41[1], f, PJ) + tfwd(a.w40[3], a.w41[3], f, PI) + tfwd(a.w40[8], a.w41[8], f, 1);
-    a.dst[2][f] += tbwd(a.w40[2], a.w41[2], f, 1) + tfwd(a.w40[5], a.w41[5], f, PI) + tfwd(a.w40[7], a.w41[7], f, PJ);
-}
-
-// Operands of the fused kernel below: lambda_V from registers, b from memory.
+// Operands of the velocity-phase bases formed from lambda_V in registers, b
+// from memory or from the staged tile.
 struct RAdjVelOps {
     const AdjVelArgs &a;
     long long e;
@@ -557,36 +754,181 @@ struct RAdjVelOps {
     __device__ __forceinline__ float lV(int c) const { return l[c]; }
     __device__ __forceinline__ float b(int c) const { return a.b[c][e]; }
 };
+struct BAdjVelOps {
+    float l[3], bb[3];
+    __device__ __forceinline__ float lV(int c) const { return l[c]; }
+    __device__ __forceinline__ float b(int c) const { return bb[c]; }
+};
 
-// lambda_V += D_V^T weights as adj_stress_gather_kernel, then, from the new
-// lambda_V of the cell, the velocity-phase weights of the next adjoint step
-// (the cell-local transpose of the velocity update, adj_vel_cell), so that
-// lambda_V is read once for both and the weights need no launch of their
-// own.  Cells of `mask` (when given: a step whose receiver residuals still
-// change their lambda_V) leave their weights to adj_source_cells_kernel.
-__global__ void __launch_bounds__(128) adj_stress_gather_vel_kernel(const GatherArgs a, const AdjVelArgs v,
-                                                                     const unsigned char *mask) {
+// lambda_V += D_V^T D, then (NEXT), from the new lambda_V of the cell, the
+// velocity-phase bases of the next adjoint step (the cell-local transpose of
+// the velocity update, adj_vel_cell), so that lambda_V is read once for both.
+// Cells of `mask` (when given: a step whose receiver residuals still change
+// their lambda_V) leave their bases to adj_source_cells_kernel.
+template <bool NEXT>
+__global__ void __launch_bounds__(128) adj_vel_kernel(const AdjGatherArgs a, const AdjVelArgs v,
+                                                      const unsigned char *mask) {
     const Geo g = a.g;
     int k, i, j;
     if (!cell_of(g, k, i, j)) return;
-    const long long f = cell_index(g, k, i, j);
-    const long long PI = g.Kp, PJ = (long long)g.Kp * g.Ip;
-    const float l0 = a.dst[0][f] + (tbwd(a.w40[0], a.w41[0], f, PI) + tfwd(a.w40[4], a.w41[4], f, PJ) +
-                                    tfwd(a.w40[6], a.w41[6], f, 1));
-    const float l1 = a.dst[1][f] + (tbwd(a.w40[1], a.w41[1], f, PJ) + tfwd(a.w40[3], a.w41[3], f, PI) +
-                                    tfwd(a.w40[8], a.w41[8], f, 1));
-    const float l2 = a.dst[2][f] + (tbwd(a.w40[2], a.w41[2], f, 1) + tfwd(a.w40[5], a.w41[5], f, PI) +
-                                    tfwd(a.w40[7], a.w41[7], f, PJ));
-    a.dst[0][f] = l0;
-    a.dst[1][f] = l1;
-    a.dst[2][f] = l2;
-    if (mask && mask[f]) return;
-    const long long col = col_index(g, i, j);
-    const bool interior = i >= v.ibk && i <= v.iek && j >= v.jbk && j <= v.jek && k <= v.kek;
-    const int s = interior ? band_sign(__ldg(&v.band[col]), k) : -1;
-    const Gb3 g0 = (interior && v.gb[0]) ? gb_load(v, f) : Gb3{};
-    const RAdjVelOps o{v, f, {l0, l1, l2}};
-    adj_vel_cell(v, o, col, k, i, j, f, s, g0);
+    const long long col = col_index(g, i, j), f = col * g.Kp + (k - 1 + KH);
+    const GCls cls{a.cls + col * a.Kc + (k - 1 + KH), a.Kc, (long long)a.Kc * g.Ip};
+    const GBase<true> D{a.D + f, g.ncell, g.Kp, (long long)g.Kp * g.Ip, cls};
+    float gv[3];
+    gather_vel(a, D, cls, gv);
+    RAdjVelOps o{v, f, {}};
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        o.l[c] = a.lV[c][f] + gv[c];
+        a.lV[c][f] = o.l[c];
+    }
+    if (!NEXT || (mask && mask[f])) return;
+    const bool interior = cls(0, 0) < 2;
+    adj_vel_cell(v, o, k, i, j, f, interior, vel_pre(v, interior, col, k, i, j, f));
+}
+
+// The staged form: lambda_V and b of a tile of 32 x 4 x 4 cells, the bases D
+// with the halos of their differences (the boxes of the forward velocity
+// update, or nine single-axis boxes near the absorber) and the classes arrive
+// by bulk tensor copies; the divergences and sums of a thread's four cells are
+// read while they travel.
+namespace adjt {
+struct VBoxes {
+    static constexpr int BJ = BJB;
+    static constexpr int n3 = 3 * BJ * BI * KT;
+    static constexpr int nI = BJ * (BI + 3) * KT, nJ = (BJ + 3) * BI * KT, nK = BJ * BI * KB;
+    static constexpr int nYZ = (BJ + 3) * BI * KB, nXZ = BJ * (BI + 3) * KB, nXY = (BJ + 3) * (BI + 3) * KT;
+    static constexpr int oB = up32(n3), oD = oB + up32(n3);
+    // shared bases: D0 i, D1 j, D2 k, D7 (yz) j k, D5 (xz) i k, D3 (xy) i j
+    static constexpr int oI = oD, oJ = oI + nI, oK = oJ + nJ, oYZ = oK + nK, oXZ = oYZ + nYZ, oXY = oXZ + nXZ;
+    static constexpr int nShared = nI + nJ + nK + nYZ + nXZ + nXY, nOwn = 3 * (nI + nJ + nK);
+    static constexpr int KC = KT + 16, nCls = (BJ + 4) * (BI + 4) * KC;
+    static constexpr int oC = oD + (nShared > nOwn ? nShared : nOwn), total = oC + up32(nCls / 4);
+    __host__ __device__ static constexpr unsigned bytes(bool touch) {
+        return 4u * (unsigned)(2 * n3 + (touch ? nOwn : nShared)) + (unsigned)nCls;
+    }
+};
+struct DShared {
+    const float *sm;
+    int tx, ty, jj;
+    using L = VBoxes;
+    // halo boxes start at -1 for the backward transposes (q 0, 1, 2), at -2 for the forward ones
+    __device__ __forceinline__ float operator()(int q, int d) const {
+        switch (q) {
+        case 0: return sm[L::oI + (jj * (BI + 3) + ty + 1 + d) * KT + tx];
+        case 1: return sm[L::oJ + ((jj + 1 + d) * BI + ty) * KT + tx];
+        case 2: return sm[L::oK + (jj * BI + ty) * KB + tx + 4 + d];
+        case 3: return sm[L::oXY + ((jj + 2) * (BI + 3) + ty + 2 + d) * KT + tx];
+        case 4: return sm[L::oXY + ((jj + 2 + d) * (BI + 3) + ty + 2) * KT + tx];
+        case 5: return sm[L::oXZ + (jj * (BI + 3) + ty + 2 + d) * KB + tx + 4];
+        case 6: return sm[L::oXZ + (jj * (BI + 3) + ty + 2) * KB + tx + 4 + d];
+        case 7: return sm[L::oYZ + ((jj + 2 + d) * BI + ty) * KB + tx + 4];
+        default: return sm[L::oYZ + ((jj + 2) * BI + ty) * KB + tx + 4 + d];
+        }
+    }
+};
+// order of the nine boxes: i: q 0 3 5; j: q 1 4 7; k: q 2 6 8
+struct DOwn {
+    const float *sm;
+    int tx, ty, jj;
+    using L = VBoxes;
+    __device__ __forceinline__ float operator()(int q, int d) const {
+        const int n = q < 3 ? 0 : (q == 3 || q == 4 || q == 6) ? 1 : 2, lo = q < 3 ? 1 : 2;
+        if (qaxis(q) == 0) return sm[L::oD + n * L::nI + (jj * (BI + 3) + ty + lo + d) * KT + tx];
+        if (qaxis(q) == 1) return sm[L::oD + 3 * L::nI + n * L::nJ + ((jj + lo + d) * BI + ty) * KT + tx];
+        return sm[L::oD + 3 * (L::nI + L::nJ) + n * L::nK + (jj * BI + ty) * KB + tx + 4 + d];
+    }
+};
+}  // namespace adjt
+
+struct VelMaps {
+    CUtensorMap own3, b3, da, db, dc, df, de, dd, cls;
+};
+
+template <bool NEXT>
+__global__ void __launch_bounds__(adjt::KT * adjt::BI, (tma::blocks_per_sm<adjt::VBoxes::total, adjt::KT * adjt::BI>()))
+    adj_vel_tma_kernel(const __grid_constant__ VelMaps tm, const __grid_constant__ AdjGatherArgs a,
+                       const __grid_constant__ AdjVelArgs v, const __grid_constant__ TmaTiles t,
+                       const unsigned char *mask) {
+    using namespace adjt;
+    using L = VBoxes;
+    constexpr int BJ = BJB;
+    extern __shared__ __align__(128) unsigned char smraw[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ unsigned long long limit;
+    float *sm = aligned128(smraw);
+    const Geo &g = a.g;
+    const Tile T = tile_of<1>(t, BI, BJ, blockIdx.x);
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const bool touch = tile_touches(a, T.k0, T.i0, T.j0, BI, BJ);
+    if (tx == 0 && ty == 0) {
+        // the copies go out first; the error word is read while they travel
+        stage_init(&bar, L::bytes(touch));
+        pdl_wait();
+        const int x0 = T.k0 - 1 + KH, ic = T.i0 + 2, jc = T.j0 + 2;
+        load_4d(sm, &tm.own3, x0, ic, jc, 0, &bar);
+        if (!touch) {
+            load_4d(sm + L::oI, &tm.da, x0, ic - 1, jc, 0, &bar);
+            load_4d(sm + L::oJ, &tm.db, x0, ic, jc - 1, 1, &bar);
+            load_4d(sm + L::oK, &tm.dc, x0 - 4, ic, jc, 2, &bar);
+            load_4d(sm + L::oYZ, &tm.df, x0 - 4, ic, jc - 2, 7, &bar);
+            load_4d(sm + L::oXZ, &tm.de, x0 - 4, ic - 2, jc, 5, &bar);
+            load_4d(sm + L::oXY, &tm.dd, x0, ic - 2, jc - 2, 3, &bar);
+        } else {
+            float *d = sm + L::oD;
+            for (int n = 0; n < 3; n++) {
+                const int lo = n == 0 ? 1 : 2;
+                load_4d(d + n * L::nI, &tm.da, x0, ic - lo, jc, n == 0 ? 0 : n == 1 ? 3 : 5, &bar);
+                load_4d(d + 3 * L::nI + n * L::nJ, &tm.db, x0, ic, jc - lo, n == 0 ? 1 : n == 1 ? 4 : 7, &bar);
+                load_4d(d + 3 * (L::nI + L::nJ) + n * L::nK, &tm.dc, x0 - 4, ic, jc, n == 0 ? 2 : n == 1 ? 6 : 8, &bar);
+            }
+        }
+        load_4d(sm + L::oB, &tm.b3, x0, ic, jc, t.f_b, &bar);
+        load_4d(sm + L::oC, &tm.cls, x0 - 8, ic - 2, jc - 2, 0, &bar);
+        limit = wait_limit(t.err);
+    }
+    const int k = T.k0 + tx, i = T.i0 + ty;
+    const bool col_ok = k <= g.nz && i <= g.nx;
+    pdl_wait();
+    pdl_launch();
+    // read while the tiles travel: the mask, and the sums and divergences or the auxiliaries of this thread's cells
+    AdjPre x[BJ];
+    bool skip[BJ];
+#pragma unroll
+    for (int jj = 0; jj < BJ; jj++) {
+        const int j = T.j0 + jj;
+        const bool interior = i >= a.ibk && i <= a.iek && j >= a.jbk && j <= a.jek && k <= a.kek;
+        const long long col = col_index(g, i, j), e = col * g.Kp + (k - 1 + KH);
+        const bool mine = NEXT && col_ok && j <= g.ny;
+        skip[jj] = mine && mask && mask[e];
+        x[jj] = mine ? vel_pre(v, interior, col, k, i, j, e) : AdjPre{};
+    }
+    __syncthreads();   // barrier initialised, wait limit set
+    const bool ok = wait_tiles(&bar, t.err, limit);
+    const unsigned char *cb = reinterpret_cast<const unsigned char *>(sm + L::oC);
+    const bool plain = !any_byte(cb, L::nCls, ty * KT + tx, KT * BI);
+    if (!ok || !col_ok) return;   // the copy failed, or no cell here
+#pragma unroll
+    for (int jj = 0; jj < BJ; jj++) {
+        const int j = T.j0 + jj;
+        if (j > g.ny) break;
+        const long long col = col_index(g, i, j), e = col * g.Kp + (k - 1 + KH);
+        const SCls<L::KC> cls{cb + ((jj + 2) * (BI + 4) + ty + 2) * L::KC + tx + 8};
+        float gv[3];
+        if (touch) gather_vel(a, DOwn{sm, tx, ty, jj}, cls, gv);
+        else if (plain) gather_vel(a, DShared{sm, tx, ty, jj}, Plain{}, gv);
+        else gather_vel(a, DShared{sm, tx, ty, jj}, cls, gv);
+        BAdjVelOps o;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            const int at = ((c * BJ + jj) * BI + ty) * KT + tx;
+            o.l[c] = sm[at] + gv[c];
+            o.bb[c] = sm[L::oB + at];
+            a.lV[c][e] = o.l[c];
+        }
+        if (!NEXT || skip[jj]) continue;
+        adj_vel_cell(v, o, k, i, j, e, plain || cls(0, 0) < 2, x[jj]);
+    }
 }
 
 // transpose of the velocity recorder (m_wav.f90:530-535): residuals as
@@ -626,10 +968,8 @@ __global__ void __launch_bounds__(128) adj_source_cells_kernel(const SrcArgs a, 
     if (!WEIGHTS || k < 1 || k > g.nz || i < 1 || i > g.nx || j < 1 || j > g.ny) return;
     const long long col = col_index(g, i, j);
     const bool interior = i >= v.ibk && i <= v.iek && j >= v.jbk && j <= v.jek && k <= v.kek;
-    const int s = interior ? band_sign(__ldg(&v.band[col]), k) : -1;
-    const Gb3 g0 = (interior && v.gb[0]) ? gb_load(v, e) : Gb3{};
     const RAdjVelOps o{v, e, {l[0], l[1], l[2]}};
-    adj_vel_cell(v, o, col, k, i, j, e, s, g0);
+    adj_vel_cell(v, o, k, i, j, e, interior, vel_pre(v, interior, col, k, i, j, e));
 }
 
 __global__ void zero_double_kernel(double *p, long long n) {
@@ -869,19 +1209,37 @@ static int adj_alloc(swpc_ctx *c) {
     for (int q = 0; q < 6; q++) s->lS[q] = s->slab + (size_t)(3 + q) * n;
     for (int comp = 0; comp < 6; comp++)
         for (int m = 0; m < c->d.nm; m++) s->lR[comp * 3 + m] = s->slab + (size_t)(9 + comp * c->d.nm + m) * n;
-    s->maps = new TmaMaps();
-    const TmaSlabs sl{s->slab, s->slab_nf, c->slab, c->slab_nf, nullptr, 0};
-    if (!tma_encode_stress(*s->maps, sl, c->g, c->d.nm, adjt::BI, adjt::BJ))
-        return set_err(c, SWPC_ERR_CUDA, "cuTensorMapEncodeTiled failed for the adjoint slab");
-    if (c->npml > 0)
-        for (int q = 0; q < 18; q++) { int rc = dalloc(c, &s->laux[q], c->npml); if (rc) return rc; }
-    for (int q = 0; q < 9; q++) {
-        int rc = dalloc(c, &s->w40[q], n);
-        if (!rc) rc = dalloc(c, &s->w41[q], n);
-        if (!rc) rc = dalloc(c, &s->w40v[q], n);
-        if (!rc) rc = dalloc(c, &s->w41v[q], n);
+    {
+        s->Kc = (c->g.Kp + 15) / 16 * 16;
+        int rc = dalloc(c, &s->U, 9 * (size_t)n);
+        if (!rc) rc = dalloc(c, &s->D, 9 * (size_t)n);
+        if (!rc) rc = dalloc(c, &s->cls, (size_t)s->Kc * c->g.Ip * c->g.Jp);
         if (rc) return rc;
     }
+    {
+        using namespace adjt;
+        constexpr int A = BJA, B = BJB;
+        AdjMaps &m = *(s->maps = new AdjMaps());
+        const Geo &g = c->g;
+        const int ns = s->slab_nf, nc = c->slab_nf;
+        auto enc = [&](unsigned char *out, float *slab, int nf, int bk, int bi, int bj, int bf) {
+            return tma_encode_box(out, slab, g, nf, bk, bi, bj, bf);
+        };
+        const bool ok = enc(m.state, s->slab, ns, KT, BI, A, 6 + 6 * c->d.nm) && enc(m.s6, s->slab, ns, KT, BI, A, 6) &&
+                        enc(m.med, c->slab, nc, KT, BI, A, 7) && enc(m.u1, s->U, 9, KB, BI + 3, A + 3, 1) &&
+                        enc(m.ui, s->U, 9, KT, BI + 3, A, 1) && enc(m.uj, s->U, 9, KT, BI, A + 3, 1) &&
+                        enc(m.uk, s->U, 9, KB, BI, A, 1) && enc(m.own3, s->slab, ns, KT, BI, B, 3) &&
+                        enc(m.b3, c->slab, nc, KT, BI, B, 3) && enc(m.da, s->D, 9, KT, BI + 3, B, 1) &&
+                        enc(m.db, s->D, 9, KT, BI, B + 3, 1) && enc(m.dc, s->D, 9, KB, BI, B, 1) &&
+                        enc(m.df, s->D, 9, KB, BI, B + 3, 1) && enc(m.de, s->D, 9, KB, BI + 3, B, 1) &&
+                        enc(m.dd, s->D, 9, KT, BI + 3, B + 3, 1) &&
+                        tma_encode_bytes(m.clsa, s->cls, s->Kc, g.Ip, g.Jp, KT + 16, BI + 4, A + 4) &&
+                        tma_encode_bytes(m.clsb, s->cls, s->Kc, g.Ip, g.Jp, KT + 16, BI + 4, B + 4);
+        if (!ok) return set_err(c, SWPC_ERR_CUDA, "cuTensorMapEncodeTiled failed for the adjoint slab");
+        m.v1[0] = 0;   // the slots, encoded with them
+    }
+    if (c->npml > 0)
+        for (int q = 0; q < 18; q++) { int rc = dalloc(c, &s->laux[q], c->npml); if (rc) return rc; }
     for (int q = 0; q < 8; q++) { int rc = dalloc(c, &s->grad[q], n); if (rc) return rc; }
     for (int q = 0; q < 8; q++) { int rc = dalloc(c, &s->gpart[q], n); if (rc) return rc; }
     return SWPC_OK;
@@ -894,10 +1252,8 @@ void adj_free(swpc_ctx *c) {
     if (s->slab) cudaFree(s->slab);   // lV, lS, lR
     delete s->maps;
     for (auto p : s->laux) if (p) cudaFree(p);
-    for (auto p : s->w40) if (p) cudaFree(p);
-    for (auto p : s->w41) if (p) cudaFree(p);
-    for (auto p : s->w40v) if (p) cudaFree(p);
-    for (auto p : s->w41v) if (p) cudaFree(p);
+    for (void *p : {(void *)s->U, (void *)s->D, (void *)s->cls})
+        if (p) cudaFree(p);
     if (s->srcmask) cudaFree(s->srcmask);
     if (s->srccells) cudaFree(s->srccells);
     for (auto p : s->grad) if (p) cudaFree(p);
@@ -924,31 +1280,52 @@ static int adj_ready(swpc_ctx *c) {
     return adj_alloc(c);
 }
 
-// staged stress-phase weights over the whole grid; fv: field of the forward V
-// in the slots buffer (gradient), or -1
-template <int NM>
+// The class of every cell; the kernel region and the band may have changed since the last call.
+static int cell_classes(swpc_ctx *c) {
+    swpc_adj_state *s = c->adj;
+    cell_class_kernel<<<148 * 8, 256, 0, c->stream>>>(c->g, c->ibk, c->iek, c->jbk, c->jek, c->kek, c->band, s->cls, s->Kc);
+    return cuda_check(c, cudaGetLastError(), "cell_class_kernel");
+}
+
+template <typename K>
+static cudaError_t smem_limit(K kernel, int bytes, unsigned long long &devices) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (devices >> dev & 1ull) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) devices |= 1ull << dev;
+    return e;
+}
+
+static const CUtensorMap &tmap(const unsigned char *p) { return *reinterpret_cast<const CUtensorMap *>(p); }
+
+// staged stress phase over the whole grid; fv: field of the forward V in the slots buffer (gradient), or -1
+template <int NM, bool GRAD>
 static cudaError_t adj_stress_tma(const swpc_adj_state *s, const AdjStrArgs &a, const TmaTiles &t, int fv,
                                   cudaStream_t st) {
     constexpr int bytes = adjt::Boxes<NM>::total * 4 + 128;
     static unsigned long long devices = 0;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!(devices >> dev & 1ull)) {
-        cudaError_t e0 = cudaFuncSetAttribute(adj_stress_tma_kernel<NM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (e0 == cudaSuccess)
-            e0 = cudaFuncSetAttribute(adj_stress_tma_kernel<NM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (e0 != cudaSuccess) return e0;
-        devices |= 1ull << dev;
-    }
-    const TmaMaps &m = *s->maps;
-    auto map = [](const unsigned char *p) -> const CUtensorMap & { return *reinterpret_cast<const CUtensorMap *>(p); };
-    const unsigned nblk = (unsigned)((long long)t.nkt * t.nit * t.njt);
-    const dim3 block(tma::KT, adjt::BI, adjt::BJ);
-    if (fv >= 0)
-        adj_stress_tma_kernel<NM, true><<<nblk, block, bytes, st>>>(map(m.state), map(m.s6), map(m.med), map(m.vh), a, t, fv);
-    else
-        adj_stress_tma_kernel<NM, false><<<nblk, block, bytes, st>>>(map(m.state), map(m.s6), map(m.med), map(m.vh), a, t, 0);
-    return cudaGetLastError();
+    const cudaError_t e = smem_limit(adj_stress_tma_kernel<NM, GRAD>, bytes, devices);
+    if (e != cudaSuccess) return e;
+    const AdjMaps &m = *s->maps;
+    const StrMaps tm{tmap(m.state), tmap(m.s6), tmap(m.med), tmap(m.v1), tmap(m.u1),
+                     tmap(m.ui),    tmap(m.uj), tmap(m.uk),  tmap(m.clsa)};
+    return launch_pdl(adj_stress_tma_kernel<NM, GRAD>, dim3((unsigned)((long long)t.nkt * t.nit * t.njt)),
+                      dim3(tma::KT, adjt::BI, adjt::BJA), bytes, st, tm, a, t, fv);
+}
+
+template <bool NEXT>
+static cudaError_t adj_vel_tma(const swpc_adj_state *s, const AdjGatherArgs &a, const AdjVelArgs &v, const TmaTiles &t,
+                               const unsigned char *mask, cudaStream_t st) {
+    constexpr int bytes = adjt::VBoxes::total * 4 + 128;
+    static unsigned long long devices = 0;
+    const cudaError_t e = smem_limit(adj_vel_tma_kernel<NEXT>, bytes, devices);
+    if (e != cudaSuccess) return e;
+    const AdjMaps &m = *s->maps;
+    const VelMaps tm{tmap(m.own3), tmap(m.b3), tmap(m.da), tmap(m.db), tmap(m.dc),
+                     tmap(m.df),   tmap(m.de), tmap(m.dd), tmap(m.clsb)};
+    return launch_pdl(adj_vel_tma_kernel<NEXT>, dim3((unsigned)((long long)t.nkt * t.nit * t.njt)),
+                      dim3(tma::KT, adjt::BI), bytes, st, tm, a, v, t, mask);
 }
 
 static SlotGeo slot_geo(const swpc_ctx *c) {
@@ -962,8 +1339,7 @@ static SlotGeo slot_geo(const swpc_ctx *c) {
     return sg;
 }
 
-// Arguments of the velocity-phase weights: from lambda_V into the
-// velocity-phase weight arrays, with the gradient of b when divS (the forward
+// Arguments of the velocity-phase bases: from lambda_V into U, with the gradient of b when divS (the forward
 // stress divergences of that step) is given.
 static AdjVelArgs vel_args(swpc_ctx *c, const float *const *divS) {
     swpc_adj_state *s = c->adj;
@@ -977,7 +1353,7 @@ static AdjVelArgs vel_args(swpc_ctx *c, const float *const *divS) {
     memcpy(a.e40, c->e40, sizeof(a.e40)); memcpy(a.e41, c->e41, sizeof(a.e41)); memcpy(a.r20, c->r20, sizeof(a.r20));
     a.dt = c->d.dt;
     a.sg = slot_geo(c);
-    for (int q = 0; q < 9; q++) { a.w40[q] = s->w40v[q]; a.w41[q] = s->w41v[q]; }
+    a.U = s->U; a.cls = s->cls; a.Kc = s->Kc;
     if (divS) {
         for (int q = 0; q < 3; q++) a.divS[q] = divS[q];
         for (int q = 0; q < 3; q++) a.gb[q] = s->gpart[5 + q];
@@ -985,88 +1361,85 @@ static AdjVelArgs vel_args(swpc_ctx *c, const float *const *divS) {
     return a;
 }
 
-// What the stress-phase gather of a step also does: form the velocity-phase
-// weights of the next adjoint step (on = true), with that step's forward
-// stress divergences divS (gradient) and leaving the cells that receiver
-// residuals change this step to the injection (skip_src).
+// What the last gather of a step also does: form the velocity-phase bases of
+// the next adjoint step (on = true), with that step's forward stress
+// divergences divS (gradient) and leaving the cells that receiver residuals
+// change this step to the injection (skip_src).
 struct AdjNext {
     bool on = false, skip_src = false;
     const float *const *divS = nullptr;
 };
 
 // one transposed step: vel^T then stress^T; with gradient when S_after /
-// V_before are given (for the staged stress-phase weights, V_before is field
-// fv of the slots buffer); vel_done: the velocity-phase weights were formed
-// by the previous step's stress-phase gather
+// V_before are given (for the staged stress phase, V_before is field fv of the
+// slots buffer); vel_done: the velocity-phase bases were formed by the
+// previous step's last gather
 static int adj_step(swpc_ctx *c, const float *const *divS_after, const float *const *V_before, int fv,
                     bool vel_done = false, const AdjNext &next = AdjNext()) {
     swpc_adj_state *s = c->adj;
     const dim3 block(kThreadsK, 2, 2);
     const dim3 grid = cell_grid(c->g, block);
     const bool grad = divS_after != nullptr;
-    {
-        if (!vel_done) {
-            // one cell per thread: the kernel is bound by its 18 weight stores, and
-            // staging its few loads (a TMA-staged form was tried) made it slower
-            adj_vel_weights_kernel<<<grid, block, 0, c->stream>>>(vel_args(c, grad ? divS_after : nullptr));
-            ACK(cudaGetLastError());
-        }
-        GatherArgs ga;
-        ga.g = c->g;
-        for (int q = 0; q < 6; q++) ga.dst[q] = s->lS[q];
-        for (int q = 0; q < 9; q++) { ga.w40[q] = s->w40v[q]; ga.w41[q] = s->w41v[q]; }
-        adj_vel_gather_kernel<<<grid, block, 0, c->stream>>>(ga);
+    const bool staged = c->adj_tma && (!grad || fv >= 0);
+    if (!vel_done) {
+        adj_vel_bases_kernel<<<grid, block, 0, c->stream>>>(vel_args(c, grad ? divS_after : nullptr));
         ACK(cudaGetLastError());
     }
-    {
-        AdjStrArgs a;
-        memset(&a, 0, sizeof(a));
-        a.g = c->g; a.ibk = c->ibk; a.iek = c->iek; a.jbk = c->jbk; a.jek = c->jek; a.kek = c->kek; a.nm = c->d.nm;
-        for (int q = 0; q < 6; q++) a.lS[q] = s->lS[q];
-        for (int q = 0; q < 18; q++) a.lR[q] = s->lR[q];
-        a.lam = c->med[1]; a.mu = c->med[2]; a.taup = c->med[3]; a.taus = c->med[4];
-        a.muyz = c->med[8]; a.muxz = c->med[9]; a.muxy = c->med[10];
-        a.band = c->band; a.pmlcol = c->pmlcol;
-        for (int q = 0; q < 9; q++) a.laV[q] = s->laux[q];
-        a.gxc = c->gx[0]; a.gxe = c->gx[1]; a.gyc = c->gy[0]; a.gye = c->gy[1]; a.gzc = c->gz[0]; a.gze = c->gz[1];
-        memcpy(a.e40, c->e40, sizeof(a.e40)); memcpy(a.e41, c->e41, sizeof(a.e41)); memcpy(a.r20, c->r20, sizeof(a.r20));
-        a.dt = c->d.dt;
-        memcpy(a.c1, c->c1, sizeof(a.c1)); memcpy(a.c2, c->c2, sizeof(a.c2)); memcpy(a.d1, c->d1, sizeof(a.d1));
-        a.d2 = c->d2;
-        a.sg = slot_geo(c);
-        for (int q = 0; q < 9; q++) { a.w40[q] = s->w40[q]; a.w41[q] = s->w41[q]; }
-        if (grad) {
-            for (int q = 0; q < 3; q++) a.V[q] = V_before[q];
-            for (int q = 0; q < 5; q++) a.gm[q] = s->gpart[q];
+    AdjStrArgs a;
+    memset(&a, 0, sizeof(a));
+    a.g = c->g; a.ibk = c->ibk; a.iek = c->iek; a.jbk = c->jbk; a.jek = c->jek; a.kek = c->kek; a.nm = c->d.nm;
+    for (int q = 0; q < 6; q++) a.lS[q] = s->lS[q];
+    for (int q = 0; q < 18; q++) a.lR[q] = s->lR[q];
+    a.lam = c->med[1]; a.mu = c->med[2]; a.taup = c->med[3]; a.taus = c->med[4];
+    a.muyz = c->med[8]; a.muxz = c->med[9]; a.muxy = c->med[10];
+    a.band = c->band; a.pmlcol = c->pmlcol;
+    for (int q = 0; q < 9; q++) a.laV[q] = s->laux[q];
+    a.gxc = c->gx[0]; a.gxe = c->gx[1]; a.gyc = c->gy[0]; a.gye = c->gy[1]; a.gzc = c->gz[0]; a.gze = c->gz[1];
+    memcpy(a.e40, c->e40, sizeof(a.e40)); memcpy(a.e41, c->e41, sizeof(a.e41)); memcpy(a.r20, c->r20, sizeof(a.r20));
+    a.dt = c->d.dt;
+    memcpy(a.c1, c->c1, sizeof(a.c1)); memcpy(a.c2, c->c2, sizeof(a.c2)); memcpy(a.d1, c->d1, sizeof(a.d1));
+    a.d2 = c->d2;
+    a.sg = slot_geo(c);
+    a.U = s->U; a.D = s->D; a.cls = s->cls; a.Kc = s->Kc;
+    if (grad) {
+        for (int q = 0; q < 3; q++) a.V[q] = V_before[q];
+        for (int q = 0; q < 5; q++) a.gm[q] = s->gpart[q];
+    }
+    if (staged) {
+        const TmaTiles t = tma_tiles(c, adjt::BI, adjt::BJA, 1, 1, kStressFields(c), 1);
+        auto run = [&](auto nm) {
+            constexpr int NM = decltype(nm)::value;
+            return grad ? adj_stress_tma<NM, true>(s, a, t, fv, c->stream) : adj_stress_tma<NM, false>(s, a, t, 0, c->stream);
+        };
+        switch (c->d.nm) {
+        case 0: ACK(run(std::integral_constant<int, 0>())); break;
+        case 1: ACK(run(std::integral_constant<int, 1>())); break;
+        case 2: ACK(run(std::integral_constant<int, 2>())); break;
+        default: ACK(run(std::integral_constant<int, 3>())); break;
         }
-        if (c->adj_tma && (!grad || fv >= 0)) {
-            const TmaTiles t = tma_tiles(c, adjt::BI, adjt::BJ, 1, 1, kStressFields(c), 1);
-            const int f = grad ? fv : -1;
-            switch (c->d.nm) {
-            case 0: ACK(adj_stress_tma<0>(s, a, t, f, c->stream)); break;
-            case 1: ACK(adj_stress_tma<1>(s, a, t, f, c->stream)); break;
-            case 2: ACK(adj_stress_tma<2>(s, a, t, f, c->stream)); break;
-            default: ACK(adj_stress_tma<3>(s, a, t, f, c->stream)); break;
-            }
-        } else {
-            switch (c->d.nm) {
-            case 0: adj_stress_weights_kernel<0><<<grid, block, 0, c->stream>>>(a); break;
-            case 1: adj_stress_weights_kernel<1><<<grid, block, 0, c->stream>>>(a); break;
-            case 2: adj_stress_weights_kernel<2><<<grid, block, 0, c->stream>>>(a); break;
-            default: adj_stress_weights_kernel<3><<<grid, block, 0, c->stream>>>(a); break;
-            }
-            ACK(cudaGetLastError());
+    } else {
+        switch (c->d.nm) {
+        case 0: adj_stress_kernel<0><<<grid, block, 0, c->stream>>>(a); break;
+        case 1: adj_stress_kernel<1><<<grid, block, 0, c->stream>>>(a); break;
+        case 2: adj_stress_kernel<2><<<grid, block, 0, c->stream>>>(a); break;
+        default: adj_stress_kernel<3><<<grid, block, 0, c->stream>>>(a); break;
         }
-        GatherArgs ga;
-        ga.g = c->g;
-        for (int q = 0; q < 3; q++) ga.dst[q] = s->lV[q];
-        for (int q = 3; q < 6; q++) ga.dst[q] = nullptr;
-        for (int q = 0; q < 9; q++) { ga.w40[q] = s->w40[q]; ga.w41[q] = s->w41[q]; }
-        if (next.on)
-            adj_stress_gather_vel_kernel<<<grid, block, 0, c->stream>>>(ga, vel_args(c, next.divS),
-                                                                         next.skip_src ? s->srcmask : nullptr);
-        else
-            adj_stress_gather_kernel<<<grid, block, 0, c->stream>>>(ga);
+        ACK(cudaGetLastError());
+    }
+    AdjGatherArgs ga;
+    memset(&ga, 0, sizeof(ga));
+    ga.g = c->g; ga.ibk = c->ibk; ga.iek = c->iek; ga.jbk = c->jbk; ga.jek = c->jek; ga.kek = c->kek;
+    for (int q = 0; q < 3; q++) ga.lV[q] = s->lV[q];
+    ga.D = s->D; ga.cls = s->cls; ga.Kc = s->Kc;
+    memcpy(ga.e40, c->e40, sizeof(ga.e40)); memcpy(ga.e41, c->e41, sizeof(ga.e41));
+    const AdjVelArgs va = vel_args(c, next.on ? next.divS : nullptr);
+    const unsigned char *mask = next.skip_src ? s->srcmask : nullptr;
+    if (staged) {
+        const TmaTiles t = tma_tiles(c, adjt::BI, adjt::BJB, 1, 1, kVelFields, 1);
+        ACK(next.on ? adj_vel_tma<true>(s, ga, va, t, mask, c->stream) : adj_vel_tma<false>(s, ga, va, t, nullptr, c->stream));
+    } else {
+        if (next.on) adj_vel_kernel<true><<<grid, block, 0, c->stream>>>(ga, va, mask);
+        else adj_vel_kernel<false><<<grid, block, 0, c->stream>>>(ga, va, nullptr);
         ACK(cudaGetLastError());
     }
     return SWPC_OK;
@@ -1203,6 +1576,7 @@ extern "C" int swpc_adj_reset(swpc_ctx *c) {
 
 extern "C" int swpc_adj_step_linear(swpc_ctx *c) {
     int rc = adj_ready(c);
+    if (!rc) rc = cell_classes(c);
     if (rc) return rc;
     rc = adj_step(c, nullptr, nullptr, -1);
     if (rc) return rc;
@@ -1450,10 +1824,10 @@ extern "C" int swpc_gradient(swpc_ctx *c, const float *obs, int ckpt, double *mi
         }
         s->ckpt = ckpt; s->nseg = nseg; s->ck_floats = ckf; s->slot_cap = cap; s->ntail = ntail;
         s->keep_floats = need_keep;
-        // the staged stress-phase weights read the forward V of a slot with its halo
+        // the staged stress phase reads the forward V of a slot with its halo
         Geo gs = c->g;
         gs.Kp = sg.Kp; gs.Ip = sg.Ip; gs.Jp = sg.Jp; gs.ncell = sg.n;
-        if (!tma_encode_box(s->maps->vh, s->slots, gs, (long long)kSlotFields * cap, tma::KB, adjt::BI + 4, adjt::BJ + 4, 3))
+        if (!tma_encode_box(s->maps->v1, s->slots, gs, (long long)kSlotFields * cap, tma::KB, adjt::BI + 3, adjt::BJA + 3, 1))
             return err(c, SWPC_ERR_CUDA, "cuTensorMapEncodeTiled failed for the recompute slots");
     }
     if (ntail > 0 && keeps_shell(c) && s->nshell != nshell) {
@@ -1513,6 +1887,7 @@ extern "C" int swpc_gradient(swpc_ctx *c, const float *obs, int ckpt, double *mi
     ACK(cudaMemcpyAsync(s->res, syn.data(), nres * sizeof(float), cudaMemcpyHostToDevice, c->stream));
     // 3. adjoint, segment by segment from the last
     rc = source_cells(c);
+    if (!rc) rc = cell_classes(c);
     if (!rc) rc = zero_adjoint(c);
     if (rc) return rc;
     for (int g = nseg - 1; g >= 0; g--) {

@@ -85,6 +85,8 @@ bool tma_encode_stress(TmaMaps &m, const TmaSlabs &s, const Geo &g, int nm, int 
 // one FP32 map (k, i, j, field) over a slab of nf fields with box (bk, bi, bj, bf)
 bool tma_encode_box(unsigned char *out, float *slab, const Geo &g, long long nf, unsigned bk, unsigned bi, unsigned bj,
                     unsigned bf);
+// a map (k, i, j) over bytes of pitch Kc (a multiple of 16), box (bk, bi, bj)
+bool tma_encode_bytes(unsigned char *out, unsigned char *p, int Kc, int Ip, int Jp, unsigned bk, unsigned bi, unsigned bj);
 bool tma_encode_vel(TmaMaps &m, const TmaSlabs &s, const Geo &g, int bi, int bj, int prec = 0);
 cudaError_t launch_stress3d_tma(const TmaMaps &m, const Str3Args &a, const TmaTiles &t, int nm, int bi, int bj, int mpc,
                                 cudaStream_t st, int prec = 0, const StressExtra &x = StressExtra());
