@@ -607,11 +607,11 @@ long long swpc_device_bytes(const swpc_ctx *ctx);
  * within a block), so that a tile's j-halo is still in L2; bi = 1 runs i then
  * j, bi = 0 (the default) takes 16 when a j plane of tiles outgrows half of
  * the L2 and 1 otherwise.
- * kernel 8 (3D) selects the stress-phase weights kernel of the adjoint step
- * (swpc_adj_*, swpc_gradient): bi = 1 the TMA-staged kernel (default), 0 the
- * one-cell-per-thread kernel.
- * kernel 9 (3D) selects how swpc_gradient forms the velocity-phase weights
- * of the adjoint step: bi = 1 (default) inside the stress-phase gather of the
+ * kernel 8 (3D) selects the kernels of the adjoint step (swpc_adj_*,
+ * swpc_gradient): bi = 1 the TMA-staged kernels (default), 0 the
+ * one-cell-per-thread kernels.
+ * kernel 9 (3D) selects how swpc_gradient forms the velocity-phase bases
+ * of the adjoint step: bi = 1 (default) inside the last gather of the
  * step before, from the lambda_V it has just summed (the cells whose
  * lambda_V receiver residuals change afterwards are formed again after the
  * injection), 0 by a kernel of their own in every step.

@@ -65,6 +65,7 @@ struct swpc_adj_state {
     int *srccells = nullptr;             // the same cells: (k, i, j) triplets, then nsrc + 1 offsets into the
                                          // contributions (station << 2 | component), in station order
     int nsrc = 0, nsrc_contrib = 0;
+    size_t srccells_cap = 0;
     double *grad[8] = {};                // lam mu muyz muxz muxy bx by bz: FP64 totals
     float *gpart[8] = {};                // the same, FP32 partial sums of the current segment
     float *res = nullptr;                // receiver residuals (nst, 3, ntw)
@@ -936,9 +937,9 @@ __global__ void __launch_bounds__(adjt::KT * adjt::BI, (tma::blocks_per_sm<adjt:
 // at j and j-1, Vz at k and k-1, the latter with the sign of an upward z), so
 // its residual r enters both; one thread per receiving cell adds the
 // residuals of its stations in station order (cells that several stations
-// share get the same bits in every run).  With WEIGHTS the thread then forms
-// the velocity-phase weights of the next adjoint step for its cell from the
-// new lambda_V (the cells the fused gather left out).
+// share get the same bits in every run).  With NEXT the thread then forms the
+// velocity-phase bases of the next adjoint step for its cell from the new
+// lambda_V (the cells the gather left out).
 struct SrcArgs {
     Geo g;
     const int *cells;       // (k, i, j) per receiving cell
@@ -950,7 +951,7 @@ struct SrcArgs {
     float *lV[3];
 };
 
-template <bool WEIGHTS>
+template <bool NEXT>
 __global__ void __launch_bounds__(128) adj_source_cells_kernel(const SrcArgs a, const AdjVelArgs v) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= a.n) return;
@@ -965,16 +966,11 @@ __global__ void __launch_bounds__(128) adj_source_cells_kernel(const SrcArgs a, 
     }
 #pragma unroll
     for (int c = 0; c < 3; c++) a.lV[c][e] = l[c];
-    if (!WEIGHTS || k < 1 || k > g.nz || i < 1 || i > g.nx || j < 1 || j > g.ny) return;
+    if (!NEXT || k < 1 || k > g.nz || i < 1 || i > g.nx || j < 1 || j > g.ny) return;
     const long long col = col_index(g, i, j);
     const bool interior = i >= v.ibk && i <= v.iek && j >= v.jbk && j <= v.jek && k <= v.kek;
     const RAdjVelOps o{v, e, {l[0], l[1], l[2]}};
     adj_vel_cell(v, o, k, i, j, e, interior, vel_pre(v, interior, col, k, i, j, e));
-}
-
-__global__ void zero_double_kernel(double *p, long long n) {
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
-        p[q] = 0.0;
 }
 
 // one slot of the recompute: the stress divergences of the interior cells,
@@ -1070,40 +1066,58 @@ struct ReconArgs {
     float *slot0;           // V of slot 0 (field c at slot0 + c * sg.n), slots every sstride floats
     size_t sstride;
 };
-__global__ void recon_kernel(const ReconArgs a) {
+// One thread per interior cell and component; the divergences of eight steps
+// are read before the first of their V is stored (the serial form, one load
+// and one store a step, took 1.20 ms for a 20-step segment of 256 x 256 x 128
+// cells).
+__global__ void __launch_bounds__(256) recon_kernel(const ReconArgs a) {
+    constexpr int U = 8;
     const int ni = a.iek - a.ibk + 1, nj = a.jek - a.jbk + 1;
     const long long n = (long long)a.kek * ni * nj;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < 3 * n;
          t += (long long)gridDim.x * blockDim.x) {
-        const int k = 1 + (int)(t % a.kek);
-        const long long r = t / a.kek;
+        const int c = (int)(t / n);
+        const long long q = t - c * n;
+        const int k = 1 + (int)(q % a.kek);
+        const long long r = q / a.kek;
         const int i = a.ibk + (int)(r % ni), j = a.jbk + (int)(r / ni);
-        const long long es = slot_index(a.sg, k, i, j), e = cell_index(a.g, k, i, j);
+        const long long es = c * a.sg.n + slot_index(a.sg, k, i, j);
+        const float b = a.b[c][cell_index(a.g, k, i, j)], dt = a.dt;
+        float v = a.slot0[es];
+        for (int m0 = 0; m0 < a.len; m0 += U) {
+            float d[U];
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-            const float b = a.b[c][e], dt = a.dt;
-            float v = a.slot0[c * a.sg.n + es];
-            for (int m = 1; m <= a.len; m++) {
-                const float d = __ldcs(a.div1 + (m - 1) * a.kstride + c * a.sg.n + es);
-                v = v + b * d * dt;
-                __stcs(a.slot0 + m * a.sstride + c * a.sg.n + es, v);
-            }
+            for (int u = 0; u < U; u++)
+                if (m0 + u < a.len) d[u] = __ldcs(a.div1 + (m0 + u) * a.kstride + es);
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (m0 + u < a.len) {
+                    v = v + b * d[u] * dt;
+                    __stcs(a.slot0 + (m0 + u + 1) * a.sstride + es, v);
+                }
         }
     }
 }
 
-// the segment's FP32 partial sums into the FP64 totals; the partials restart from zero
+// the segment's FP32 partial sums into the FP64 totals, over the interior
+// cells (the only ones that have sums); the partials restart from zero.  One
+// warp per column of the region.
 struct FoldArgs {
     double *total[8];
     float *part[8];
 };
-__global__ void fold_gradient_kernel(const FoldArgs a, long long n) {
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+__global__ void __launch_bounds__(256) fold_gradient_kernel(const FoldArgs a, Geo g, int ibk, int iek, int jbk, int jek,
+                                                            int kek) {
+    const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+    const int ni = iek - ibk + 1, ncol = ni * (jek - jbk + 1);
+    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < ncol; w += nw) {
+        const long long e0 = cell_index(g, 1, ibk + w % ni, jbk + w / ni);
+        for (int k = lane; k < kek; k += 32)
 #pragma unroll
-        for (int f = 0; f < 8; f++) {
-            a.total[f][q] += (double)a.part[f][q];
-            a.part[f][q] = 0.0f;
-        }
+            for (int f = 0; f < 8; f++) {
+                a.total[f][e0 + k] += (double)a.part[f][e0 + k];
+                a.part[f][e0 + k] = 0.0f;
+            }
     }
 }
 
@@ -1123,8 +1137,9 @@ struct ModelGradArgs {
     Geo g;
     const double *gm[8];           // lam mu muyz muxz muxy bx by bz
     const float *lam, *mu, *b[3];  // relaxed medium, buoyancies
-    const float *vp, *vs, *rho;    // the model (device layout)
-    double *out[3];                // d misfit / d vp, vs, rho
+    const float *vp, *vs, *rho;    // the model, a memory box of leading extents ld_k, ld_i
+    double *out[3];                // d misfit / d vp, vs, rho, likewise
+    int ld_k, ld_i;
 };
 
 // sum over the four entries of a 4-point harmonic mean that contain cell e
@@ -1156,11 +1171,8 @@ __device__ double hmean_adjoint(const double *gf, const float *mu, long long e, 
     return acc;
 }
 
-__global__ void __launch_bounds__(128) model_grad_kernel(const ModelGradArgs a) {
-    const Geo g = a.g;
-    int k, i, j;
-    if (!cell_of(g, k, i, j)) return;
-    const long long e = cell_index(g, k, i, j);
+// cell e of the device layout, h of the model's box
+__device__ __forceinline__ void model_grad_cell(const ModelGradArgs &a, const Geo &g, long long e, long long h) {
     const long long PI = g.Kp, PJ = (long long)g.Kp * g.Ip;
     const double glam = a.gm[0][e];
     const double gmu = a.gm[1][e] + hmean_adjoint(a.gm[2], a.mu, e, 1, PJ) + hmean_adjoint(a.gm[3], a.mu, e, 1, PI) +
@@ -1173,11 +1185,28 @@ __global__ void __launch_bounds__(128) model_grad_kernel(const ModelGradArgs a) 
         grho += a.gm[5 + q][e] * (-0.5 * b0 * b0) + a.gm[5 + q][e - boff[q]] * (-0.5 * b1 * b1);
     }
     const double lam = a.lam[e], mu = a.mu[e];
-    const double vp = a.vp[e], vs = a.vs[e], rho = a.rho[e];
+    const double vp = a.vp[h], vs = a.vs[h], rho = a.rho[h];
     const double m2 = lam + 2.0 * mu;
-    a.out[0][e] = vp > 0.0 ? glam * 2.0 * m2 / vp : 0.0;
-    a.out[1][e] = vs > 0.0 ? (gmu - 2.0 * glam) * 2.0 * mu / vs : 0.0;
-    a.out[2][e] = grho + (rho > 0.0 ? (glam * lam + gmu * mu) / rho : 0.0);
+    a.out[0][h] = vp > 0.0 ? glam * 2.0 * m2 / vp : 0.0;
+    a.out[1][h] = vs > 0.0 ? (gmu - 2.0 * glam) * 2.0 * mu / vs : 0.0;
+    a.out[2][h] = grho + (rho > 0.0 ? (glam * lam + gmu * mu) / rho : 0.0);
+}
+
+// one warp per column of the memory box; the cells outside the grid get zeros
+__global__ void __launch_bounds__(256) model_grad_kernel(const ModelGradArgs a) {
+    const Geo g = a.g;
+    const int col = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), nib = g.nx + 6;
+    if (col >= nib * (g.ny + 6)) return;
+    const int i = col % nib - 2, j = col / nib - 2;
+    const bool in = i >= 1 && i <= g.nx && j >= 1 && j <= g.ny;
+    for (int k = (int)(threadIdx.x & 31) - 2; k <= g.nz + 3; k += 32) {
+        const long long h = ((long long)(j + 2) * a.ld_i + (i + 2)) * a.ld_k + (k + 2);
+        if (in && k >= 1 && k <= g.nz) {
+            model_grad_cell(a, g, cell_index(g, k, i, j), h);
+        } else {
+            for (int q = 0; q < 3; q++) a.out[q][h] = 0.0;
+        }
+    }
 }
 
 dim3 cell_grid(const Geo &g, dim3 block) {
@@ -1238,10 +1267,16 @@ static int adj_alloc(swpc_ctx *c) {
         if (!ok) return set_err(c, SWPC_ERR_CUDA, "cuTensorMapEncodeTiled failed for the adjoint slab");
         m.v1[0] = 0;   // the slots, encoded with them
     }
-    if (c->npml > 0)
-        for (int q = 0; q < 18; q++) { int rc = dalloc(c, &s->laux[q], c->npml); if (rc) return rc; }
-    for (int q = 0; q < 8; q++) { int rc = dalloc(c, &s->grad[q], n); if (rc) return rc; }
-    for (int q = 0; q < 8; q++) { int rc = dalloc(c, &s->gpart[q], n); if (rc) return rc; }
+    // the auxiliaries, sums and totals in one block each: one memset clears them
+    int rc = c->npml > 0 ? dalloc(c, &s->laux[0], 18 * (size_t)c->npml) : 0;
+    if (!rc) rc = dalloc(c, &s->grad[0], 8 * (size_t)n);
+    if (!rc) rc = dalloc(c, &s->gpart[0], 8 * (size_t)n);
+    if (rc) return rc;
+    for (int q = 1; q < 18 && s->laux[0]; q++) s->laux[q] = s->laux[0] + q * c->npml;
+    for (int q = 1; q < 8; q++) {
+        s->grad[q] = s->grad[0] + q * n;
+        s->gpart[q] = s->gpart[0] + q * n;
+    }
     return SWPC_OK;
 }
 
@@ -1251,13 +1286,13 @@ void adj_free(swpc_ctx *c) {
     if (!s) return;
     if (s->slab) cudaFree(s->slab);   // lV, lS, lR
     delete s->maps;
-    for (auto p : s->laux) if (p) cudaFree(p);
+    if (s->laux[0]) cudaFree(s->laux[0]);
     for (void *p : {(void *)s->U, (void *)s->D, (void *)s->cls})
         if (p) cudaFree(p);
     if (s->srcmask) cudaFree(s->srcmask);
     if (s->srccells) cudaFree(s->srccells);
-    for (auto p : s->grad) if (p) cudaFree(p);
-    for (auto p : s->gpart) if (p) cudaFree(p);
+    if (s->grad[0]) cudaFree(s->grad[0]);
+    if (s->gpart[0]) cudaFree(s->gpart[0]);
     if (s->res) cudaFree(s->res);
     if (s->ckpool) cudaFree(s->ckpool);
     if (s->slots) cudaFree(s->slots);
@@ -1454,8 +1489,8 @@ static bool source_at(const swpc_ctx *c, int it) {
 }
 
 // residuals of step it into lambda_V; with divS_next (the fused path) the
-// receiving cells also form the velocity-phase weights of step it - 1
-static int adj_source(swpc_ctx *c, int it, const float *const *divS_next = nullptr, bool weights = false) {
+// receiving cells also form the velocity-phase bases of step it - 1
+static int adj_source(swpc_ctx *c, int it, const float *const *divS_next = nullptr, bool bases = false) {
     swpc_adj_state *s = c->adj;
     if (!source_at(c, it) || s->nsrc <= 0) return SWPC_OK;
     SrcArgs a;
@@ -1471,7 +1506,7 @@ static int adj_source(swpc_ctx *c, int it, const float *const *divS_next = nullp
     a.scale = 0.5f * c->M0 * c->UC * 1e9f;
     for (int q = 0; q < 3; q++) a.lV[q] = s->lV[q];
     const unsigned nb = (unsigned)((s->nsrc + 127) / 128);
-    if (weights) adj_source_cells_kernel<true><<<nb, 128, 0, c->stream>>>(a, vel_args(c, divS_next));
+    if (bases) adj_source_cells_kernel<true><<<nb, 128, 0, c->stream>>>(a, vel_args(c, divS_next));
     else adj_source_cells_kernel<false><<<nb, 128, 0, c->stream>>>(a, AdjVelArgs{});
     return cuda_check(c, cudaGetLastError(), "adj_source_cells_kernel");
 }
@@ -1512,7 +1547,6 @@ static int source_cells(swpc_ctx *c) {
     std::vector<int> packed(cells);
     packed.insert(packed.end(), offs.begin(), offs.end());
     packed.insert(packed.end(), contrib.begin(), contrib.end());
-    if (s->srccells) { cudaFree(s->srccells); s->srccells = nullptr; }
     s->nsrc = s->nsrc_contrib = 0;
     if (!s->srcmask && cudaMalloc((void **)&s->srcmask, (size_t)g.ncell) != cudaSuccess) {
         cudaGetLastError();
@@ -1521,7 +1555,13 @@ static int source_cells(swpc_ctx *c) {
     }
     ACK(cudaMemsetAsync(s->srcmask, 0, (size_t)g.ncell, c->stream));
     if (ncell > 0) {
-        ACK(cudaMalloc((void **)&s->srccells, packed.size() * sizeof(int)));
+        if (s->srccells_cap < packed.size()) {
+            if (s->srccells) cudaFree(s->srccells);
+            s->srccells = nullptr;
+            s->srccells_cap = 0;
+            ACK(cudaMalloc((void **)&s->srccells, packed.size() * sizeof(int)));
+            s->srccells_cap = packed.size();
+        }
         ACK(cudaMemcpyAsync(s->srccells, packed.data(), packed.size() * sizeof(int), cudaMemcpyHostToDevice,
                             c->stream));
         s->nsrc = ncell;
@@ -1535,23 +1575,18 @@ static int source_cells(swpc_ctx *c) {
 
 static int zero_adjoint(swpc_ctx *c) {
     swpc_adj_state *s = c->adj;
-    const size_t n = sizeof(float) * c->g.ncell;
-    for (auto p : s->lV) if (p) ACK(cudaMemsetAsync(p, 0, n, c->stream));
-    for (auto p : s->lS) if (p) ACK(cudaMemsetAsync(p, 0, n, c->stream));
-    for (auto p : s->lR) if (p) ACK(cudaMemsetAsync(p, 0, n, c->stream));
-    for (auto p : s->laux) if (p) ACK(cudaMemsetAsync(p, 0, sizeof(float) * c->npml, c->stream));
-    for (auto p : s->grad) {
-        zero_double_kernel<<<148 * 4, 256, 0, c->stream>>>(p, c->g.ncell);
-        ACK(cudaGetLastError());
-    }
-    for (auto p : s->gpart) ACK(cudaMemsetAsync(p, 0, n, c->stream));
+    const size_t n = (size_t)c->g.ncell;
+    ACK(cudaMemsetAsync(s->slab, 0, s->slab_nf * n * sizeof(float), c->stream));   // lV, lS, lR
+    if (s->laux[0]) ACK(cudaMemsetAsync(s->laux[0], 0, 18 * c->npml * sizeof(float), c->stream));
+    ACK(cudaMemsetAsync(s->grad[0], 0, 8 * n * sizeof(double), c->stream));
+    ACK(cudaMemsetAsync(s->gpart[0], 0, 8 * n * sizeof(float), c->stream));
     return SWPC_OK;
 }
 
 static int fold_gradient(swpc_ctx *c) {
     FoldArgs a;
     for (int q = 0; q < 8; q++) { a.total[q] = c->adj->grad[q]; a.part[q] = c->adj->gpart[q]; }
-    fold_gradient_kernel<<<148 * 4, 256, 0, c->stream>>>(a, c->g.ncell);
+    fold_gradient_kernel<<<148 * 8, 256, 0, c->stream>>>(a, c->g, c->ibk, c->iek, c->jbk, c->jek, c->kek);
     return cuda_check(c, cudaGetLastError(), "fold_gradient_kernel");
 }
 
@@ -1616,7 +1651,19 @@ static std::vector<float *> state_arrays(swpc_ctx *c, std::vector<size_t> *sizes
         if (c->R[q]) { v.push_back(c->R[q]); sizes->push_back(c->g.ncell); }
     if (c->npml > 0)
         for (int q = 0; q < 18; q++) { v.push_back(c->aux[q]); sizes->push_back(c->npml); }
-    return v;
+    // arrays that follow one another are one range (the field slab; the auxiliaries)
+    std::vector<float *> runs;
+    std::vector<size_t> len;
+    for (size_t n = 0; n < v.size(); n++) {
+        if (!runs.empty() && v[n] == runs.back() + len.back()) {
+            len.back() += (*sizes)[n];
+            continue;
+        }
+        runs.push_back(v[n]);
+        len.push_back((*sizes)[n]);
+    }
+    *sizes = len;
+    return runs;
 }
 
 static int copy_state(swpc_ctx *c, float *ck, bool save) {
@@ -1632,7 +1679,7 @@ static int copy_state(swpc_ctx *c, float *ck, bool save) {
 }
 
 // Slot `slot` of the recompute: V over the slot box (read with its halo by
-// the stress-phase weights) and the stress divergences of the interior cells
+// the adjoint stress phase) and the stress divergences of the interior cells
 // (the velocity-phase gradient), kSlotFields fields in the slot layout.
 constexpr int kSlotFields = 6;
 static int save_slot(swpc_ctx *c, int slot) {
@@ -1930,7 +1977,7 @@ extern "C" int swpc_gradient(swpc_ctx *c, const float *obs, int ckpt, double *mi
             const float *base = kept ? kept_step(it) : s->slots + (size_t)(it - it0 + 1) * slot_floats + 3 * n;
             for (int q = 0; q < 3; q++) D[q] = base + q * n;
         };
-        // within a segment each stress-phase gather also forms the velocity-phase weights of the step before
+        // within a segment the last gather of each step also forms the velocity-phase bases of the step before
         // (kernel 9 of swpc_set_launch); the first step of a segment forms its own
         bool vel_done = false;
         for (int it = it1; it >= it0 && !rc; it--) {
@@ -1975,19 +2022,6 @@ extern "C" int swpc_gradient_fetch(swpc_ctx *c, int which, double *out, int ld_k
     return fetch_double(c, c->adj->grad[which], out, ld_k, ld_i);
 }
 
-// device double array -> device memory box (leading extents ld_k, ld_i)
-__global__ void unpack_double_kernel(Geo g, const double *__restrict__ src, double *dst, int ld_k, int ld_i) {
-    const int nkb = g.nz + 6, nib = g.nx + 6;
-    const long long n = (long long)nkb * nib * (g.ny + 6);
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int kb = (int)(t % nkb);
-        const long long col = t / nkb;
-        const int ib = (int)(col % nib), jb = (int)(col / nib);
-        dst[((long long)jb * ld_i + ib) * ld_k + kb] = src[cell_index(g, kb - 2, ib - 2, jb - 2)];
-    }
-}
-
 static bool is_device_array(const void *p) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
@@ -2021,41 +2055,58 @@ static int gradient_model(swpc_ctx *c, const float *vp, const float *vs, const f
     const Geo &g = c->g;
     if (ld_k < g.nz + 6 || ld_i < g.nx + 6) return err(c, SWPC_ERR_ARG, "leading extents smaller than the memory box");
     ACK(cudaSetDevice(c->device));
-    float *dm[3] = {};
-    double *dg[3] = {};
-    int rc = SWPC_OK;
-    const float *hm[3] = {vp, vs, rho};
-    for (int q = 0; q < 3 && !rc; q++) {
-        rc = dalloc(c, &dm[q], g.ncell);
-        if (!rc) rc = dalloc(c, &dg[q], g.ncell);
-        if (!rc) rc = on_device ? copy_box_from_device(c, dm[q], hm[q], ld_k, ld_i)
-                                : copy_box(c, dm[q], hm[q], nullptr, ld_k, ld_i);
+    ModelGradArgs a;
+    a.g = g;
+    for (int q = 0; q < 8; q++) a.gm[q] = c->adj->grad[q];
+    a.lam = c->med[1]; a.mu = c->med[2];
+    for (int q = 0; q < 3; q++) a.b[q] = c->med[5 + q];
+    const unsigned nb = (unsigned)(((long long)(g.nx + 6) * (g.ny + 6) + 7) / 8);
+    if (on_device) {
+        // the caller's arrays are read and written in place
+        a.vp = vp; a.vs = vs; a.rho = rho;
+        a.out[0] = gvp; a.out[1] = gvs; a.out[2] = grho;
+        a.ld_k = ld_k; a.ld_i = ld_i;
+        model_grad_kernel<<<nb, 256, 0, c->stream>>>(a);
+        ACK(cudaGetLastError());
+        return cuda_check(c, cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
     }
+    // host arrays through a box without padding on the device
+    const int nk = g.nz + 6, ni = g.nx + 6;
+    const size_t ncol = (size_t)ni * (g.ny + 6), n = ncol * nk;
+    float *dm = nullptr;
+    double *dg = nullptr;
+    if (cudaMalloc((void **)&dm, 3 * n * sizeof(float)) != cudaSuccess ||
+        cudaMalloc((void **)&dg, 3 * n * sizeof(double)) != cudaSuccess) {
+        cudaGetLastError();
+        if (dm) cudaFree(dm);
+        return err(c, SWPC_ERR_NOMEM, "no room for the model gradient");
+    }
+    a.vp = dm; a.vs = dm + n; a.rho = dm + 2 * n;
+    for (int q = 0; q < 3; q++) a.out[q] = dg + q * n;
+    a.ld_k = nk; a.ld_i = ni;
+    const float *hm[3] = {vp, vs, rho};
+    double *ho[3] = {gvp, gvs, grho};
+    std::vector<double> h(n);
+    int rc = SWPC_OK;
+    for (int q = 0; q < 3 && !rc; q++)
+        for (int j = 0; j < g.ny + 6 && !rc; j++)
+            rc = cuda_check(c, cudaMemcpy2DAsync(dm + q * n + (size_t)j * ni * nk, nk * sizeof(float),
+                                                 hm[q] + (size_t)j * ld_i * ld_k, ld_k * sizeof(float),
+                                                 nk * sizeof(float), ni, cudaMemcpyHostToDevice, c->stream),
+                            "cudaMemcpy2DAsync");
     if (!rc) {
-        ModelGradArgs a;
-        a.g = g;
-        for (int q = 0; q < 8; q++) a.gm[q] = c->adj->grad[q];
-        a.lam = c->med[1]; a.mu = c->med[2];
-        for (int q = 0; q < 3; q++) a.b[q] = c->med[5 + q];
-        a.vp = dm[0]; a.vs = dm[1]; a.rho = dm[2];
-        for (int q = 0; q < 3; q++) a.out[q] = dg[q];
-        const dim3 block(kThreadsK, 2, 2);
-        model_grad_kernel<<<cell_grid(g, block), block, 0, c->stream>>>(a);
+        model_grad_kernel<<<nb, 256, 0, c->stream>>>(a);
         rc = cuda_check(c, cudaGetLastError(), "model_grad_kernel");
     }
-    double *ho[3] = {gvp, gvs, grho};
     for (int q = 0; q < 3 && !rc; q++) {
-        if (on_device) {
-            unpack_double_kernel<<<148 * 8, 256, 0, c->stream>>>(g, dg[q], ho[q], ld_k, ld_i);
-            rc = cuda_check(c, cudaGetLastError(), "unpack_double_kernel");
-        } else {
-            rc = fetch_double(c, dg[q], ho[q], ld_k, ld_i);
-        }
+        rc = cuda_check(c, cudaMemcpyAsync(h.data(), dg + q * n, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream),
+                        "cudaMemcpyAsync");
+        if (!rc) rc = cuda_check(c, cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
+        for (size_t r = 0; r < ncol && !rc; r++)
+            memcpy(ho[q] + ((r / ni) * ld_i + r % ni) * ld_k, h.data() + r * nk, nk * sizeof(double));
     }
     cudaStreamSynchronize(c->stream);
-    for (int q = 0; q < 3; q++) {
-        if (dm[q]) { cudaFree(dm[q]); c->bytes -= (long long)g.ncell * sizeof(float); }
-        if (dg[q]) { cudaFree(dg[q]); c->bytes -= (long long)g.ncell * sizeof(double); }
-    }
+    cudaFree(dm);
+    cudaFree(dg);
     return rc;
 }

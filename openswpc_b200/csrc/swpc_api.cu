@@ -250,6 +250,8 @@ extern "C" int swpc_destroy(swpc_ctx *c) {
     for (auto p : c->S) if (p) cudaFree(p);
     for (auto p : c->R) if (p) cudaFree(p);
     for (auto p : c->med) if (p) cudaFree(p);
+    if (is3d(c))   // aux[0] owns the block
+        for (int q = 1; q < 18; q++) c->aux[q] = nullptr;
     for (auto p : c->aux) if (p) cudaFree(p);
     for (int q = 0; q < 2; q++) {
         if (c->gx[q]) cudaFree(c->gx[q]);
@@ -286,13 +288,13 @@ extern "C" int swpc_set_launch(swpc_ctx *c, int kernel, int minb, int bi, int bj
         return SWPC_OK;
     }
     if (kernel == 8) {
-        // adjoint stress-phase weights: bi = 1 staged, 0 one cell per thread
+        // adjoint step: bi = 1 staged kernels, 0 one cell per thread
         if (!is3d(c) || (bi != 0 && bi != 1)) return set_err(c, SWPC_ERR_ARG, "kernel 8 (3D): bi = 0 or 1");
         c->adj_tma = bi == 1;
         return SWPC_OK;
     }
     if (kernel == 9) {
-        // adjoint velocity-phase weights: bi = 1 formed by the stress-phase gather of the step before (the
+        // velocity-phase bases of the adjoint: bi = 1 formed by the last gather of the step before (the
         // gradient's default), 0 by their own kernel
         if (!is3d(c) || (bi != 0 && bi != 1)) return set_err(c, SWPC_ERR_ARG, "kernel 9 (3D): bi = 0 or 1");
         c->adj_fuse = bi == 1;
@@ -674,10 +676,12 @@ extern "C" int swpc_absorb_setup(swpc_ctx *c, const float *gxc, const float *gxe
             base += (len + 7) / 8 * 8;
         }
     c->npml = base;
-    for (int q = 0; q < 18; q++) {
-        if (c->aux[q]) { cudaFree(c->aux[q]); c->aux[q] = nullptr; }
-        RC(dalloc(c, &c->aux[q], (size_t)std::max<long long>(base, 1)));
-    }
+    // one block, aux[0] the owner
+    const long long len = std::max<long long>(base, 1);
+    if (c->aux[0]) cudaFree(c->aux[0]);
+    for (auto &p : c->aux) p = nullptr;
+    RC(dalloc(c, &c->aux[0], 18 * (size_t)len));
+    for (int q = 1; q < 18; q++) c->aux[q] = c->aux[0] + q * len;
     CK(cudaMemcpyAsync(c->pmlcol, pc.data(), ncol * sizeof(int2), cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     c->absorb_ready = true;

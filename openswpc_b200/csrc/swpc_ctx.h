@@ -207,8 +207,8 @@ struct swpc_ctx {
     // (swpc2d_tma.cu): tiles 32 x 16 with stress_tbi / vel_tbi threads along i
     bool stress_tma = false, vel_tma = false;
     int stress_tbi = 4, stress_tbj = 4, vel_tbi = 4, vel_tbj = 4;
-    bool adj_tma = true;          // staged stress-phase adjoint weights (swpc_adjoint.cu)
-    bool adj_fuse = true;         // velocity-phase adjoint weights formed by the stress-phase gather before
+    bool adj_tma = true;          // staged adjoint kernels (swpc_adjoint.cu)
+    bool adj_fuse = true;         // velocity-phase adjoint bases formed by the gather before
     float *div_out = nullptr;     // the gradient's kept step: the velocity update stores the stress divergences here
     int div_geo[4] = {0, 0, 0, 0};   // its layout: Kp, Ip, i0, j0 (Vel3Args divo)
     long long div_n = 0;

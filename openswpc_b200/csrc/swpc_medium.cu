@@ -482,9 +482,8 @@ extern "C" int swpc_medium_setup_device_opt(swpc_ctx *c, float fq_min, float fq_
     CK(cudaGetLastError());
     band_kernel<<<kGrid, kBlock, 0, c->stream>>>(g, c->kfs, c->kob, c->band);
     CK(cudaGetLastError());
-    // the two words of the velocity range reduction
-    unsigned *d_mm = nullptr;
-    CK(cudaMalloc((void **)&d_mm, 2 * sizeof(unsigned)));
+    // the two words of the velocity range reduction (the report's, which clears them before each use)
+    unsigned *const d_mm = c->vmax_buf;
     const unsigned init[2] = {0u, 0xffffffffu};
     unsigned mm[2] = {0u, 0xffffffffu};
     int rc = cuda_check(c, cudaMemcpyAsync(d_mm, init, sizeof(init), cudaMemcpyHostToDevice, c->stream),
@@ -510,7 +509,6 @@ extern "C" int swpc_medium_setup_device_opt(swpc_ctx *c, float fq_min, float fq_
     }
     if (!rc) rc = average_medium(c);
     if (!rc) rc = cuda_check(c, cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
-    cudaFree(d_mm);
     if (rc) return rc;
     float vmax1 = -1.0f, vmin1 = 1e30f;
     if (mm[0] != 0u) {
