@@ -242,14 +242,20 @@ struct Aux9 {
     long long q;   // index of the cell in the compact arrays (without the member offset)
     float v[9];
 };
-__device__ __forceinline__ Aux9 aux_load(float *const *aux, long long ao, const int2 *pmlcol, const Geo &g, int k,
-                                         int i, int j) {
+__device__ __forceinline__ Aux9 aux_load_at(float *const *aux, long long ao, long long q) {
     Aux9 r;
-    const int2 pc = __ldg(&pmlcol[col_index(g, i, j)]);
-    r.q = (long long)pc.y + (k - pc.x);
+    r.q = q;
 #pragma unroll
     for (int n = 0; n < 9; n++) r.v[n] = lds(&aux[n][ao + r.q]);
     return r;
+}
+__device__ __forceinline__ int aux_index(const int2 *pmlcol, const Geo &g, int k, int i, int j) {
+    const int2 pc = __ldg(&pmlcol[col_index(g, i, j)]);
+    return pc.y + (k - pc.x);
+}
+__device__ __forceinline__ Aux9 aux_load(float *const *aux, long long ao, const int2 *pmlcol, const Geo &g, int k,
+                                         int i, int j) {
+    return aux_load_at(aux, ao, aux_index(pmlcol, g, k, i, j));
 }
 
 template <int PREC, class Ops>

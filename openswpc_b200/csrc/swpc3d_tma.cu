@@ -342,8 +342,25 @@ __global__ void __launch_bounds__(KT * BI, (blocks_per_sm<VelBoxes<BI, BJ, M, PR
     }
     pdl_wait();
     pdl_launch();
-    constexpr bool PRE = BJ * M <= 2;
-    Aux9 xs[PRE ? M : 1][PRE ? BJ : 1];
+    // Two cells' auxiliaries are in flight at a time (a single member walks
+    // down its BJ planes): all four at once do not fit the registers of six
+    // CTAs per SM (76 bytes spilled, 5 % slower), and loading each cell's
+    // after the tile wait left the absorber waiting four times a tile (192 x
+    // 192 x 96 cells, half of them absorber: 76.1 us, now 70.1 us).
+    constexpr bool PRE = BJ * M <= 2, WALK = M == 1 && BJ > 2 && PREC == PREC_F32;
+    Aux9 xs[PRE ? M : 1][PRE ? BJ : WALK ? 2 : 1];
+    int aq[WALK ? BJ : 1];   // place of an absorber cell's auxiliaries, -1 for the others
+    if (WALK) {
+#pragma unroll
+        for (int jj = 0; jj < BJ; jj++) {
+            const int j = T.j0 + jj;
+            const bool interior = i >= a.ibk && i <= a.iek && j >= a.jbk && j <= a.jek && k <= a.kek;
+            aq[WALK ? jj : 0] = (col_ok && j <= g.ny && !interior && (a.mask & 2)) ? aux_index(a.pmlcol, g, k, i, j) : -1;
+        }
+#pragma unroll
+        for (int jj = 0; jj < 2; jj++)
+            if (aq[WALK ? jj : 0] >= 0) xs[0][WALK ? jj : 0] = aux_load_at(a.aS, (long long)T.m0 * t.ao, aq[WALK ? jj : 0]);
+    }
     if (PRE && col_ok && (a.mask & 2)) {
 #pragma unroll
         for (int mm = 0; mm < (PRE ? M : 1); mm++)
@@ -365,15 +382,17 @@ __global__ void __launch_bounds__(KT * BI, (blocks_per_sm<VelBoxes<BI, BJ, M, PR
             const int j = T.j0 + jj;
             if (j > g.ny) break;
             const bool interior = i >= a.ibk && i <= a.iek && j >= a.jbk && j <= a.jek && k <= a.kek;
-            if (!(a.mask & (interior ? 1 : 2))) continue;
             const SVelOps<BI, BJ, PREC> o{sm + L::oMem(mm), sm, tx, ty, jj, a};
             const long long e = col_index(g, i, j) * g.Kp + (k - 1 + KH);
-            if (interior) {
+            if (interior && (a.mask & 1)) {
                 vel_interior<PREC>(a, o, sgn[jj], a.Vx + so, a.Vy + so, a.Vz + so, e);
-            } else {
-                const Aux9 ax = PRE ? xs[PRE ? mm : 0][PRE ? jj : 0] : aux_load(a.aS, ao, a.pmlcol, g, k, i, j);
+            } else if (!interior && (a.mask & 2)) {
+                const Aux9 ax = PRE ? xs[PRE ? mm : 0][PRE ? jj : 0]
+                              : WALK ? xs[0][WALK ? jj & 1 : 0] : aux_load(a.aS, ao, a.pmlcol, g, k, i, j);
                 vel_absorber<PREC>(a, o, ax, k, i, j, e, ao, a.Vx + so, a.Vy + so, a.Vz + so);
             }
+            if (WALK && jj + 2 < BJ)
+                if (aq[WALK ? jj + 2 : 0] >= 0) xs[0][WALK ? jj & 1 : 0] = aux_load_at(a.aS, ao, aq[WALK ? jj + 2 : 0]);
             if (src[jj] >= 0) inject_cell(x.inj, x.d_it ? *x.d_it : x.it, src[jj], e);   // single members only
         }
     }
