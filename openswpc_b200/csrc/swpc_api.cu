@@ -157,6 +157,7 @@ extern "C" int swpc_create(const swpc_desc *d, swpc_ctx **out) {
             // the TMA-staged kernels are the default launch of FP32 3D contexts
             c->stress_tma = true;
             c->vel_tma = true;
+            c->stress_tbj = c->vel_tbj = staged_planes(g, 1);
         }
         const long long ncol = (long long)g.Ip * g.Jp;
         if (!rc) rc = dalloc(c, &c->band, ncol);

@@ -64,8 +64,13 @@ struct swpc_fbatch {
     bool src_dirty = true;
     int strip = 0;                 // i-strip width in cells (0: automatic), flat kernels
     bool staged = false;           // TMA-staged kernels (FP32 contexts with a field slab)
-    int sbi = 4, sbj = 2, smpc = 2, vbi = 4, vbj = 2, vmpc = 2;   // staged tiles and members per CTA
-    int tiles_first = 0;           // staged launch order (see swpc3d_tma.cu tile_of)
+    // staged tiles and members per CTA, and launch order (tile_of): one member
+    // per CTA, tiles fastest (9 members of 144 x 160 x 80 cells 1013 us a step,
+    // two members a CTA on 32 x 4 x 2 tiles 1082 us; 6 of 256 x 256 x 128 2830
+    // against 2922 us): a CTA of two members saves medium bytes but leaves
+    // fewer CTAs, hence fewer copies in flight
+    int sbi = 4, sbj = 4, smpc = 1, vbi = 4, vbj = 4, vmpc = 1;
+    int tiles_first = 1;
     void *tmaps = nullptr;         // swpc::TmaMaps over the batch slab and the context's medium
     int tma_key[4] = {-1, -1, -1, -1};
     int *d_it = nullptr;
@@ -220,6 +225,7 @@ extern "C" int swpc_fbatch_create(swpc_ctx *c, int nmem, swpc_fbatch **out) {
         for (int comp = 0; comp < 6; comp++)
             for (int m = 0; m < c->d.nm; m++) b->R[comp * 3 + m] = F(9 + comp * c->d.nm + m);
         b->staged = c->slab != nullptr;
+        b->sbj = b->vbj = staged_planes(c->g, nmem);
     }
     if (c->npml > 0)
         for (int q = 0; q < 18 && !rc; q++) rc = falloc(b, &b->aux[q], (size_t)c->npml * nmem);

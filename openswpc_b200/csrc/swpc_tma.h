@@ -49,6 +49,18 @@ struct TmaTiles {
 // the j-block length); the field indices follow the context's slab
 TmaTiles tma_tiles(const swpc_ctx *c, int bi, int bj, int nmem, int mpc, int nfields, int live);
 
+// Tile planes bj (32 x 4 x bj cells) of the staged FP32 kernels for a launch of
+// nmem members: 2 below 6,000 tiles of four planes, where the larger CTAs
+// leave too few rounds per SM (stress + velocity with 2 against 4 planes: 128 x
+// 128 x 40 cells 49.9 against 53.7 us, 128 x 128 x 100 112.5 against 118.5 us; a
+// 40 x 36 x 32 shot of 60 steps 1.17 against 1.31 ms), 4 above, where their
+// smaller halos win (200 steps of 192 x 192 x 96 48.3 against 47.8 ms, 256 x 256 x
+// 128 465 against 462 us, 9 members of 144 x 160 x 80 1050 against 1013 us).
+inline int staged_planes(const Geo &g, int nmem) {
+    const long long tiles = (long long)((g.nz + 31) / 32) * ((g.nx + 3) / 4) * ((g.ny + 3) / 4) * nmem;
+    return tiles < 6000 ? 2 : 4;
+}
+
 // fields a staged stress / velocity update reads over its tile (member state
 // and medium): S, R, V, lam mu taup taus muyz muxz muxy, bx by bz / V, S, bx by bz
 inline int kStressFields(const swpc_ctx *c) { return 16 + 6 * c->d.nm; }
