@@ -92,13 +92,14 @@ int slab_fields2d(int kind, int nm);
 bool staged2d_ti_ok(int ti);
 bool encode_maps2d(Maps2D &m, int kind, int nm, float *slab, const Geo &g);
 // one launch over the ntiles tiles from `tiles`, all of models model0 ..
-// model0 + nset - 1 (nset = 1 .. kGroup2D), whose map sets are sets[0 .. nset-1]
+// model0 + nset - 1 (nset = 1 .. kGroup2D), whose map sets are sets[0 .. nset-1];
+// a single run hands its descriptor over on the host (one)
 cudaError_t launch_stress2d_tma(int kind, int nm, int ti, const MapSet2D *sets, int nset, int model0,
                                 const Model2D *models, const Tile2D *tiles, int ntiles, int mask, Fields2D f, int *err,
-                                cudaStream_t st, const Step2D &x = Step2D());
+                                cudaStream_t st, const Step2D &x = Step2D(), const Model2D *one = nullptr);
 cudaError_t launch_vel2d_tma(int kind, int ti, const MapSet2D *sets, int nset, int model0, const Model2D *models,
                              const Tile2D *tiles, int ntiles, int mask, Fields2D f, int *err, cudaStream_t st,
-                             const Step2D &x = Step2D());
+                             const Step2D &x = Step2D(), const Model2D *one = nullptr);
 // flags of the tile (k0, i0) of a model (tile extents 32 x ni)
 int tile2d_flags(const swpc_ctx *c, int k0, int i0, int ni);
 

@@ -86,7 +86,13 @@ int create_2d(swpc_ctx *c) {
     if (!encode_maps2d(*mp, c->kind, nm, c->slab, g))
         return set_err(c, SWPC_ERR_CUDA, "cuTensorMapEncodeTiled failed for the 2D field slab");
     c->stress_tma = c->vel_tma = true;
-    c->stress_tbi = c->vel_tbi = 8;
+    // 16 threads along i (one row each) up to three tiles per SM, where a
+    // tile's own time counts, 8 beyond, where more tiles fit an SM (16 against
+    // 8, us a step: P-SV 256 x 128 7.4 against 9.2, 700 x 300 10.1 against 13.3,
+    // SH 256 x 128 6.2 against 7.2; P-SV 1024 x 512 19.0 against 17.0, 2048 x
+    // 1024 73.8 against 67.5)
+    const long long tiles = (long long)((g.nz + 31) / 32) * ((g.nx + kTileI2D - 1) / kTileI2D);
+    c->stress_tbi = c->vel_tbi = tiles <= 3 * 148 ? 16 : 8;
     return build_tiles_2d(c);
 }
 
@@ -302,10 +308,11 @@ int update_stress_2d(swpc_ctx *c, int mask, const Step2D &x) {
 
 int update_stress_2d_kernel(swpc_ctx *c, int mask, const Step2D &x) {
     const int m = (c->d.na > 0 && c->abc == 0) ? mask : (mask & 1);
+    const Model2D one = model_of(c);
     if (c->stress_tma)
         return cuda_check(c, launch_stress2d_tma(c->kind, c->d.nm, c->stress_tbi, &static_cast<Maps2D *>(c->maps2d)->str,
                                                  1, 0, c->d_model2d, c->d_tiles2d, c->ntiles2d, m,
-                                                 fields2d(c->kind, c->d.nm), c->d_err, c->stream, x),
+                                                 fields2d(c->kind, c->d.nm), c->d_err, c->stream, x, &one),
                           "stress2d_tma launch");
     launch_stress2d(c->kind, c->d.nm, c->d_model2d, c->d_tiles2d, c->ntiles2d, m, kDefaultTiles, c->stream);
     return cuda_check(c, cudaGetLastError(), "stress2d launch");
@@ -322,10 +329,11 @@ int update_vel_2d(swpc_ctx *c, int mask, const Step2D &x) {
 
 int update_vel_2d_kernel(swpc_ctx *c, int mask, const Step2D &x) {
     const int m = (c->d.na > 0 && c->abc == 0) ? mask : (mask & 1);
+    const Model2D one = model_of(c);
     if (c->vel_tma)
         return cuda_check(c, launch_vel2d_tma(c->kind, c->vel_tbi, &static_cast<Maps2D *>(c->maps2d)->vel, 1, 0,
                                               c->d_model2d, c->d_tiles2d, c->ntiles2d, m, fields2d(c->kind, c->d.nm),
-                                              c->d_err, c->stream, x),
+                                              c->d_err, c->stream, x, &one),
                           "vel2d_tma launch");
     launch_vel2d(c->kind, c->d_model2d, c->d_tiles2d, c->ntiles2d, m, kDefaultTiles, c->stream);
     return cuda_check(c, cudaGetLastError(), "vel2d launch");

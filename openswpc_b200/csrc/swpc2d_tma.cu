@@ -51,14 +51,27 @@ constexpr int KM = KT + 4;    // k extent of a box over k0 .. k0+35 (mu, rho)
 enum { ST_STATE, ST_S, ST_MED, ST_MU, ST_V };
 enum { VE_OWN, VE_RHO, VE_A, VE_C, VE_E };
 
-// the maps of the G models of a launch (kernel parameter)
+// the maps of the G models of a launch (kernel parameter); a single run's model
+// descriptor travels with them
 template <int G>
 struct MapGroup {
     MapSet2D set[G];
 };
+template <>
+struct MapGroup<1> {
+    MapSet2D set[1];
+    Model2D model;
+};
 
 __device__ __forceinline__ const CUtensorMap *set_maps(const MapSet2D &s) {
     return reinterpret_cast<const CUtensorMap *>(&s);
+}
+
+// Minimum resident CTAs a kernel is compiled for: a batch's 8-thread form keeps
+// n by its registers (24 uneven P-SV models: 191 us a step, 197 us without).
+template <int TI, int G>
+constexpr int min_ctas(int n) {
+    return G > 1 && TI == 8 ? n : 1;
 }
 
 // the block's copy of the model descriptor
@@ -67,6 +80,20 @@ __device__ __forceinline__ void copy_model(const Model2D *__restrict__ models, i
     const int *src = reinterpret_cast<const int *>(models + model);
     int *dst = reinterpret_cast<int *>(&sM);
     for (int w = threadIdx.y * blockDim.x + threadIdx.x; w < nw; w += blockDim.x * blockDim.y) dst[w] = __ldg(src + w);
+}
+
+// A batch's CTA copies its model's descriptor to shared memory; a single run
+// reads the parameter (no loads, and the band signs wait for no barrier).
+template <int G>
+struct ModelCopy {
+    Model2D m;
+};
+template <>
+struct ModelCopy<1> {};
+template <int G>
+__device__ __forceinline__ const Model2D &model_in(const MapGroup<G> &pm, const ModelCopy<G> &c) {
+    if constexpr (G > 1) return c.m;
+    else return pm.model;
 }
 
 // ---------------------------------------------------------------------------
@@ -149,7 +176,7 @@ __device__ __noinline__ void record(const Step2D &x, int cta) {
 }
 
 template <int KIND, int NM, int TI, int G>
-__global__ void __launch_bounds__(32 * TI) stress2d_tma_kernel(const __grid_constant__ MapGroup<G> pm, int model0,
+__global__ void __launch_bounds__(32 * TI, min_ctas<TI, G>(5)) stress2d_tma_kernel(const __grid_constant__ MapGroup<G> pm, int model0,
                                                                const Model2D *__restrict__ models,
                                                                const Tile2D *__restrict__ tiles, int mask,
                                                                Fields2D f, int *err,
@@ -157,7 +184,7 @@ __global__ void __launch_bounds__(32 * TI) stress2d_tma_kernel(const __grid_cons
     using L = StrBox<KIND, NM>;
     constexpr int RI = BI / TI;
     extern __shared__ __align__(128) unsigned char smraw[];
-    __shared__ Model2D sM;
+    __shared__ ModelCopy<G> sM;
     __shared__ __align__(8) uint64_t bar;
     __shared__ unsigned long long limit;
     float *sm = aligned128(smraw);
@@ -188,11 +215,11 @@ __global__ void __launch_bounds__(32 * TI) stress2d_tma_kernel(const __grid_cons
         load_3d(sm + L::oV, &mp[ST_V], x0 - 4, ic - 2, f.v, &bar);
         limit = wait_limit(err);
     }
-    copy_model(models, tl.model, sM);
+    if constexpr (G > 1) copy_model(models, tl.model, sM.m);
     pdl_wait();
     pdl_launch();
     __syncthreads();   // barrier initialised, wait limit and model descriptor set
-    const Model2D &M = sM;
+    const Model2D &M = model_in(pm, sM);
     // the band signs and source columns of this thread's cells are read while the tiles travel
     const int *icol = x.inj ? x.inj[tl.model].col : nullptr;
     int sg[RI], src[RI];
@@ -225,14 +252,14 @@ __global__ void __launch_bounds__(32 * TI) stress2d_tma_kernel(const __grid_cons
 }
 
 template <int KIND, int TI, int G>
-__global__ void __launch_bounds__(32 * TI) vel2d_tma_kernel(const __grid_constant__ MapGroup<G> pm, int model0,
+__global__ void __launch_bounds__(32 * TI, min_ctas<TI, G>(6)) vel2d_tma_kernel(const __grid_constant__ MapGroup<G> pm, int model0,
                                                             const Model2D *__restrict__ models,
                                                             const Tile2D *__restrict__ tiles, int mask, Fields2D f,
                                                             int *err, int *it_next) {
     using L = VelBox<KIND>;
     constexpr int RI = BI / TI;
     extern __shared__ __align__(128) unsigned char smraw[];
-    __shared__ Model2D sM;
+    __shared__ ModelCopy<G> sM;
     __shared__ __align__(8) uint64_t bar;
     __shared__ unsigned long long limit;
     float *sm = aligned128(smraw);
@@ -265,11 +292,11 @@ __global__ void __launch_bounds__(32 * TI) vel2d_tma_kernel(const __grid_constan
         }
         limit = wait_limit(err);
     }
-    copy_model(models, tl.model, sM);
+    if constexpr (G > 1) copy_model(models, tl.model, sM.m);
     pdl_wait();
     pdl_launch();
     __syncthreads();   // barrier initialised, wait limit and model descriptor set
-    const Model2D &M = sM;
+    const Model2D &M = model_in(pm, sM);
     // the band signs of this thread's cells are read while the tiles travel
     int sg[RI];
 #pragma unroll
@@ -309,6 +336,7 @@ cudaError_t smem_attr(K kernel, int bytes, unsigned long long &devices) {
 struct MapArgs {
     const MapSet2D *sets;
     int nset, model0;
+    const Model2D *one;   // host descriptor of a single run
 };
 
 template <int G>
@@ -316,6 +344,7 @@ MapGroup<G> group_of(const MapArgs &ma) {
     MapGroup<G> g;
     memset(&g, 0, sizeof(g));
     for (int q = 0; q < ma.nset && q < G; q++) g.set[q] = ma.sets[q];
+    if constexpr (G == 1) g.model = *ma.one;
     return g;
 }
 
@@ -344,7 +373,7 @@ cudaError_t run_vel(const MapArgs &ma, const Model2D *models, const Tile2D *tile
 template <int KIND, int NM, int TI>
 cudaError_t stress_g(const MapArgs &ma, const Model2D *models, const Tile2D *tiles, int ntiles, int mask, Fields2D f,
                      int *err, cudaStream_t st, const Step2D &x) {
-    if (ma.nset > 1) return run_stress<KIND, NM, TI, kGroup2D>(ma, models, tiles, ntiles, mask, f, err, st, x);
+    if (!ma.one) return run_stress<KIND, NM, TI, kGroup2D>(ma, models, tiles, ntiles, mask, f, err, st, x);
     return run_stress<KIND, NM, TI, 1>(ma, models, tiles, ntiles, mask, f, err, st, x);
 }
 
@@ -370,7 +399,7 @@ cudaError_t stress_nm(int nm, int ti, const MapArgs &ma, const Model2D *models, 
 template <int KIND, int TI>
 cudaError_t vel_g(const MapArgs &ma, const Model2D *models, const Tile2D *tiles, int ntiles, int mask, Fields2D f,
                   int *err, cudaStream_t st, const Step2D &x) {
-    if (ma.nset > 1) return run_vel<KIND, TI, kGroup2D>(ma, models, tiles, ntiles, mask, f, err, st, x);
+    if (!ma.one) return run_vel<KIND, TI, kGroup2D>(ma, models, tiles, ntiles, mask, f, err, st, x);
     return run_vel<KIND, TI, 1>(ma, models, tiles, ntiles, mask, f, err, st, x);
 }
 
@@ -438,19 +467,20 @@ bool encode_maps2d(Maps2D &m, int kind, int nm, float *slab, const Geo &g) {
 
 cudaError_t launch_stress2d_tma(int kind, int nm, int ti, const MapSet2D *sets, int nset, int model0,
                                 const Model2D *models, const Tile2D *tiles, int ntiles, int mask, Fields2D f, int *err,
-                                cudaStream_t st, const Step2D &x) {
+                                cudaStream_t st, const Step2D &x, const Model2D *one) {
     if (ntiles <= 0) return cudaSuccess;
     if (nset < 1 || nset > kGroup2D) return cudaErrorInvalidValue;
-    const MapArgs ma{sets, nset, model0};
+    const MapArgs ma{sets, nset, model0, one};
     if (kind == SWPC_KIND_PSV) return stress_nm<0>(nm, ti, ma, models, tiles, ntiles, mask, f, err, st, x);
     return stress_nm<1>(nm, ti, ma, models, tiles, ntiles, mask, f, err, st, x);
 }
 
 cudaError_t launch_vel2d_tma(int kind, int ti, const MapSet2D *sets, int nset, int model0, const Model2D *models,
-                             const Tile2D *tiles, int ntiles, int mask, Fields2D f, int *err, cudaStream_t st, const Step2D &x) {
+                             const Tile2D *tiles, int ntiles, int mask, Fields2D f, int *err, cudaStream_t st, const Step2D &x,
+                             const Model2D *one) {
     if (ntiles <= 0) return cudaSuccess;
     if (nset < 1 || nset > kGroup2D) return cudaErrorInvalidValue;
-    const MapArgs ma{sets, nset, model0};
+    const MapArgs ma{sets, nset, model0, one};
     if (kind == SWPC_KIND_PSV) return vel_ti<0>(ti, ma, models, tiles, ntiles, mask, f, err, st, x);
     return vel_ti<1>(ti, ma, models, tiles, ntiles, mask, f, err, st, x);
 }
