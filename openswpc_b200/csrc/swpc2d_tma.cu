@@ -67,11 +67,13 @@ __device__ __forceinline__ const CUtensorMap *set_maps(const MapSet2D &s) {
     return reinterpret_cast<const CUtensorMap *>(&s);
 }
 
-// Minimum resident CTAs a kernel is compiled for: a batch's 8-thread form keeps
-// n by its registers (24 uneven P-SV models: 191 us a step, 197 us without).
-template <int TI, int G>
+// Resident CTAs the 8-thread P-SV kernels are compiled for, stress and velocity
+// (0: the compiler's choice of 54 and 44 registers): with 4 and 5, 64 and 48
+// registers, a 256 x 128 model takes 8.0 instead of 9.2 us a step, 1024 x 512
+// 16.8 instead of 18.3, 24 uneven models 190 instead of 197; SH kernels lose 5 %.
+template <int KIND, int TI>
 constexpr int min_ctas(int n) {
-    return G > 1 && TI == 8 ? n : 1;
+    return KIND == 0 && TI == 8 ? n : 0;
 }
 
 // the block's copy of the model descriptor
@@ -85,14 +87,8 @@ __device__ __forceinline__ void copy_model(const Model2D *__restrict__ models, i
 // A batch's CTA copies its model's descriptor to shared memory; a single run
 // reads the parameter (no loads, and the band signs wait for no barrier).
 template <int G>
-struct ModelCopy {
-    Model2D m;
-};
-template <>
-struct ModelCopy<1> {};
-template <int G>
-__device__ __forceinline__ const Model2D &model_in(const MapGroup<G> &pm, const ModelCopy<G> &c) {
-    if constexpr (G > 1) return c.m;
+__device__ __forceinline__ const Model2D &model_in(const MapGroup<G> &pm, const Model2D &copy) {
+    if constexpr (G > 1) return copy;
     else return pm.model;
 }
 
@@ -176,7 +172,7 @@ __device__ __noinline__ void record(const Step2D &x, int cta) {
 }
 
 template <int KIND, int NM, int TI, int G>
-__global__ void __launch_bounds__(32 * TI, min_ctas<TI, G>(5)) stress2d_tma_kernel(const __grid_constant__ MapGroup<G> pm, int model0,
+__global__ void __launch_bounds__(32 * TI, min_ctas<KIND, TI>(4)) stress2d_tma_kernel(const __grid_constant__ MapGroup<G> pm, int model0,
                                                                const Model2D *__restrict__ models,
                                                                const Tile2D *__restrict__ tiles, int mask,
                                                                Fields2D f, int *err,
@@ -184,7 +180,7 @@ __global__ void __launch_bounds__(32 * TI, min_ctas<TI, G>(5)) stress2d_tma_kern
     using L = StrBox<KIND, NM>;
     constexpr int RI = BI / TI;
     extern __shared__ __align__(128) unsigned char smraw[];
-    __shared__ ModelCopy<G> sM;
+    __shared__ Model2D sM;   // batches
     __shared__ __align__(8) uint64_t bar;
     __shared__ unsigned long long limit;
     float *sm = aligned128(smraw);
@@ -215,7 +211,7 @@ __global__ void __launch_bounds__(32 * TI, min_ctas<TI, G>(5)) stress2d_tma_kern
         load_3d(sm + L::oV, &mp[ST_V], x0 - 4, ic - 2, f.v, &bar);
         limit = wait_limit(err);
     }
-    if constexpr (G > 1) copy_model(models, tl.model, sM.m);
+    if constexpr (G > 1) copy_model(models, tl.model, sM);
     pdl_wait();
     pdl_launch();
     __syncthreads();   // barrier initialised, wait limit and model descriptor set
@@ -252,14 +248,14 @@ __global__ void __launch_bounds__(32 * TI, min_ctas<TI, G>(5)) stress2d_tma_kern
 }
 
 template <int KIND, int TI, int G>
-__global__ void __launch_bounds__(32 * TI, min_ctas<TI, G>(6)) vel2d_tma_kernel(const __grid_constant__ MapGroup<G> pm, int model0,
+__global__ void __launch_bounds__(32 * TI, min_ctas<KIND, TI>(5)) vel2d_tma_kernel(const __grid_constant__ MapGroup<G> pm, int model0,
                                                             const Model2D *__restrict__ models,
                                                             const Tile2D *__restrict__ tiles, int mask, Fields2D f,
                                                             int *err, int *it_next) {
     using L = VelBox<KIND>;
     constexpr int RI = BI / TI;
     extern __shared__ __align__(128) unsigned char smraw[];
-    __shared__ ModelCopy<G> sM;
+    __shared__ Model2D sM;   // batches
     __shared__ __align__(8) uint64_t bar;
     __shared__ unsigned long long limit;
     float *sm = aligned128(smraw);
@@ -292,7 +288,7 @@ __global__ void __launch_bounds__(32 * TI, min_ctas<TI, G>(6)) vel2d_tma_kernel(
         }
         limit = wait_limit(err);
     }
-    if constexpr (G > 1) copy_model(models, tl.model, sM.m);
+    if constexpr (G > 1) copy_model(models, tl.model, sM);
     pdl_wait();
     pdl_launch();
     __syncthreads();   // barrier initialised, wait limit and model descriptor set
