@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(KT * BI, (blocks_per_sm<VelBoxes<BI, BJ, M, PR
     __shared__ unsigned long long limit;
     float *sm = aligned128(smraw);
     const Geo g = a.g;
-    const Tile T = tile_of<M>(t, BI, BJ, blockIdx.x);
+    const Tile T = tile_of<M>(t, BI, BJ, t.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
     const int tx = threadIdx.x, ty = threadIdx.y;
     const bool lead = tx == 0 && ty == 0;
     if (x.it_next && lead && blockIdx.x == 0) {

@@ -606,6 +606,7 @@ struct Boxes {
     // one component with the halo of its three differences; one operator's halo in i, j or k
     static constexpr int n1 = up32((BJ + 3) * (BI + 3) * KB);
     static constexpr int nI = BJ * (BI + 3) * KT, nJ = (BJ + 3) * BI * KT, nK = BJ * BI * KB;
+    static_assert(nI % 32 == 0 && nJ % 32 == 0 && nK % 32 == 0, "every box starts on a 128-byte boundary");
     static constexpr int nU = 3 * n1 > 3 * (nI + nJ + nK) ? 3 * n1 : 3 * (nI + nJ + nK);
     static constexpr int KC = KT + 16, nCls = (BJ + 4) * (BI + 4) * KC;   // bytes
     static constexpr int oState = up32(nMed), oU = oState + up32(nState), oV = oU + up32(nU), oC = oV + 3 * n1,
@@ -805,6 +806,8 @@ struct VBoxes {
     static constexpr int nShared = nI + nJ + nK + nYZ + nXZ + nXY, nOwn = 3 * (nI + nJ + nK);
     static constexpr int KC = KT + 16, nCls = (BJ + 4) * (BI + 4) * KC;
     static constexpr int oC = oD + (nShared > nOwn ? nShared : nOwn), total = oC + up32(nCls / 4);
+    static_assert(nI % 32 == 0 && nJ % 32 == 0 && nK % 32 == 0 && nYZ % 32 == 0 && nXZ % 32 == 0,
+                  "every box starts on a 128-byte boundary");
     __host__ __device__ static constexpr unsigned bytes(bool touch) {
         return 4u * (unsigned)(2 * n3 + (touch ? nOwn : nShared)) + (unsigned)nCls;
     }
@@ -859,7 +862,7 @@ __global__ void __launch_bounds__(adjt::KT * adjt::BI, (tma::blocks_per_sm<adjt:
     __shared__ unsigned long long limit;
     float *sm = aligned128(smraw);
     const Geo &g = a.g;
-    const Tile T = tile_of<1>(t, BI, BJ, blockIdx.x);
+    const Tile T = tile_of<1>(t, BI, BJ, t.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
     const int tx = threadIdx.x, ty = threadIdx.y;
     const bool touch = tile_touches(a, T.k0, T.i0, T.j0, BI, BJ);
     if (tx == 0 && ty == 0) {
@@ -1470,7 +1473,8 @@ static int adj_step(swpc_ctx *c, const float *const *divS_after, const float *co
     const AdjVelArgs va = vel_args(c, next.on ? next.divS : nullptr);
     const unsigned char *mask = next.skip_src ? s->srcmask : nullptr;
     if (staged) {
-        const TmaTiles t = tma_tiles(c, adjt::BI, adjt::BJB, 1, 1, kVelFields, 1);
+        TmaTiles t = tma_tiles(c, adjt::BI, adjt::BJB, 1, 1, kVelFields, 1);
+        t.rev = reverse_tiles(c->g, c->slab_nf);
         ACK(next.on ? adj_vel_tma<true>(s, ga, va, t, mask, c->stream) : adj_vel_tma<false>(s, ga, va, t, nullptr, c->stream));
     } else {
         if (next.on) adj_vel_kernel<true><<<grid, block, 0, c->stream>>>(ga, va, mask);

@@ -1155,6 +1155,7 @@ TmaTiles tma_tiles(const swpc_ctx *c, int bi, int bj, int nmem, int mpc, int nfi
     t.nmem = nmem;
     t.mgroups = (nmem + mpc - 1) / mpc;
     t.tiles_first = 0;
+    t.rev = 0;
     // launch order: blocks of j tiles once a j plane of tiles (the fields the
     // kernel reads over bj planes, for the members whose tiles interleave in
     // the launch order) outgrows half of the L2
@@ -1272,7 +1273,8 @@ static int launch_vel_kernel(swpc_ctx *c, int mask, const VelExtra &x) {
     a.scale = c->d_scale;
     if (c->vel_tma && c->slab) {
         RC(tma_ready(c));
-        const TmaTiles t = tma_tiles(c, c->vel_tbi, c->vel_tbj, 1, 1, kVelFields, 1);
+        TmaTiles t = tma_tiles(c, c->vel_tbi, c->vel_tbj, 1, 1, kVelFields, 1);
+        t.rev = reverse_tiles(c->g, c->slab_nf);
         return cuda_check(c, launch_vel3d_tma(*static_cast<TmaMaps *>(c->tmaps), a, t, c->vel_tbi, c->vel_tbj, 1,
                                               c->stream, c->prec, x), "vel3d_tma launch");
     }

@@ -31,6 +31,7 @@ struct TmaTiles {
     int nkt, nit, njt;
     int nmem, mgroups;   // members, groups of members per CTA
     int tiles_first;     // launch order: 0 member groups fastest, 1 tiles fastest
+    int rev;             // tiles in reverse order (velocity-phase launches, see reverse_tiles)
     int jblock;          // tiles of a group: k fastest, then blocks of jblock j tiles (j, then i)
     int f_v;             // state slab: Vx of member 0 (S follows at f_v + 3)
     int f_state;         // state slab: Sxx of member 0 (S, then R)
@@ -65,6 +66,18 @@ inline int staged_planes(const Geo &g, int nmem) {
 // and medium): S, R, V, lam mu taup taus muyz muxz muxy, bx by bz / V, S, bx by bz
 inline int kStressFields(const swpc_ctx *c) { return 16 + 6 * c->d.nm; }
 constexpr int kVelFields = 12;
+
+// Whether velocity-phase launches run their tiles backwards: the stress phase
+// ends with the last tiles' V and S in L2, where the velocity phase then
+// starts, and the other way round.  That pays where the step's fields outgrow
+// the 126 MB of L2 but not by much (192 x 192 x 96 cells, 0.65 GB: 217.3 us a
+// step, backwards 213.0; 128 x 128 x 100 120.3 and 118.0; 256 x 256 x 128, 1.5
+// GB: 495.5 and 492.2); within it (96 x 96 x 64) forward order is 2 % faster,
+// and at 512 x 512 x 256 0.3 %.
+inline int reverse_tiles(const Geo &g, int nfields) {
+    const double bytes = 4.0 * nfields * g.ncell;
+    return bytes > 126e6 && bytes < 2e9;
+}
 
 // the slabs the tensor maps cover
 struct TmaSlabs {
