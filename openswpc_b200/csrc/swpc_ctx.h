@@ -237,6 +237,8 @@ struct swpc_ctx {
 // helpers shared by the translation units
 namespace swpc {
 int set_err(swpc_ctx *c, int code, const std::string &msg);
+// drops the captured steps (every graph of the context): after any setup change (swpc_api.cu)
+int graph_invalidate(swpc_ctx *c);
 // 2 na must fit the grid across x and y (the whole grid for a block of a
 // decomposed one); refused when the medium arrives
 int upload_scales(swpc_ctx *c);   // swpc_api.cu

@@ -162,11 +162,7 @@ extern "C" int swpc_green_store_setup(swpc_ctx *c, int ng, const int *ig, const 
         ijk[3 * n] = ig[n]; ijk[3 * n + 1] = jg[n]; ijk[3 * n + 2] = kg[n];
     }
     CK(cudaSetDevice(c->device));
-    c->desc_dirty = true;
-    if (c->graph_exec) {
-        cudaGraphExecDestroy(c->graph_exec);
-        c->graph_exec = nullptr;
-    }
+    graph_invalidate(c);
     green_free(c);
     if (ng == 0) return SWPC_OK;
     const int ncmp = bforce ? 9 : 6;

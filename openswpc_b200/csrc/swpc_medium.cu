@@ -49,13 +49,7 @@ struct KRow {
                 // 3 seawater (0 <= z < depth(1); p0 holds its lam)
 };
 
-void drop_graph(swpc_ctx *c) {
-    c->desc_dirty = true;
-    if (c->graph_exec) {
-        cudaGraphExecDestroy(c->graph_exec);
-        c->graph_exec = nullptr;
-    }
-}
+void drop_graph(swpc_ctx *c) { graph_invalidate(c); }
 
 // the memory box k, i, j in [-2, n+3] of the grid-stride index q
 __device__ __forceinline__ void box_cell(const Geo &g, long long q, int &k, int &i, int &j) {

@@ -128,10 +128,6 @@ extern "C" int swpc_set_pw_mode(swpc_ctx *c, int on) {
     if (on && (c->g.nx < 2 || c->g.ny < 2)) return set_err(c, SWPC_ERR_ARG, "the plane-wave mode needs nx, ny >= 2");
     if (on && c->sub) return set_err(c, SWPC_ERR_ARG, "the plane-wave mode runs on a single domain");
     c->pw_mode = on ? 1 : 0;
-    c->desc_dirty = true;
-    if (c->graph_exec) {
-        cudaGraphExecDestroy(c->graph_exec);
-        c->graph_exec = nullptr;
-    }
+    graph_invalidate(c);
     return SWPC_OK;
 }

@@ -100,3 +100,30 @@ def test_step2d(kind, dims, nsrc, nst, nt):
         for x, y in zip(out(runs[0]), single[0]):
             assert _same(x, y)
         b.close()
+
+
+@pytest.mark.parametrize("what", ["green_store", "medium"])
+def test_setup_between_runs(what):
+    """A setup change between two runs of whole step graphs reaches the second one."""
+    p = small3d(nx=33, ny=29, nz=30, na=4, nt=40)
+    out = []
+    for graphs in (True, False):
+        r = Swpc3D(p, medium_on_device=True)
+
+        def steps(it0):
+            if graphs:
+                r.run(it0, 20)
+            else:
+                for it in range(it0, it0 + 20):
+                    r.step(it)
+        steps(1)
+        if what == "green_store":
+            r.green_store_setup([10, 20], [9, 21], [8, 12])
+        else:
+            xi = np.full((p.ny + 6, p.nx + 6, p.nz + 6), 0.05, np.float32)
+            r.medium.__init__(r.lib, r.ctx, p, xi)
+        steps(21)
+        out.append([r.waveforms(), r.download(_lib.F_VZ)] + ([r.green_functions()] if what == "green_store" else []))
+        r.close()
+    for a, b in zip(*out):
+        assert np.abs(b).max() > 0 and _same(a, b)
