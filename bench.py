@@ -100,14 +100,14 @@ B_PSV_INT, B_PSV_PML = 38 * 4, 34 * 4
 # (stress 0.941 + 0.546 GB, velocity 0.328 + 0.087 GB against 1.481 + 0.430 GB; the 2D batch summary under profiles/)
 TRAFFIC_PER_ALGORITHMIC_2D = (0.941275 + 0.545625 + 0.328020 + 0.086632) / (1.4813472 + 0.429801472)
 # one adjoint step per cell (FP32 state, FP32 segment sums of the gradients, nm = 3), interior / absorber:
-# velocity weights (lV, b read, nine w40 + nine w41 written, the three stress divergences of the slot read, three b
-# gradient sums read and written; absorber: nine PML auxiliaries read and written instead of the divergences and
-# sums), velocity gather (18 weights read, six lS read and written), stress weights (lS, seven medium fields, 18 lR
-# read and written, 18 weights written, V of the slot, five medium gradient sums read and written; absorber: lS,
-# five medium fields, nine auxiliaries, 18 weights), stress gather (18 weights read, three lV read and written)
-B_ADJ_INT = (12 + 12 + 72 + 12 + 24) + (72 + 48) + (24 + 28 + 144 + 72 + 12 + 40) + (72 + 24)
-B_ADJ_PML = (12 + 12 + 72 + 72) + (72 + 48) + (24 + 20 + 72 + 72) + (72 + 24)
-# inside a checkpoint segment the stress gather of each step forms the velocity weights of the next from the lV it
+# velocity bases (lV, b read, three bases written, the three stress divergences of the slot read, three b gradient
+# sums read and written; absorber: nine PML auxiliaries read and written and nine bases), stress phase (the bases
+# read, lS and 18 lR read and written, seven medium fields, six bases written, V of the slot, five medium gradient
+# sums read and written; absorber: nine bases read and nine written, lS, five medium fields, nine auxiliaries),
+# velocity gather (the stress-phase bases read, three lV read and written)
+B_ADJ_INT = (12 + 12 + 12 + 12 + 24) + (12 + 48 + 144 + 28 + 24 + 12 + 40) + (24 + 24)
+B_ADJ_PML = (12 + 12 + 36 + 72) + (36 + 48 + 20 + 72 + 36) + (36 + 24)
+# inside a checkpoint segment the velocity gather of each step forms the velocity bases of the next from the lV it
 # has just summed, so every step but the first of a segment reads lV once instead of twice
 B_ADJ_FUSED_SAVES = 12
 # every forward step whose slot is kept or recomputed: V copied into the slot over the kernel region with a two-cell
@@ -728,9 +728,10 @@ def bench_c3(args, world, rank, local):
                     "d2h_bytes_per_step": d2h,
                     "what": "waveform_misfit(vp, vs, rho) + backward from CPU tensors: medium setup on the host, "
                             "upload, gradient, chain rule, gradients back, wall clock"},
-            # per gradient: forward and recompute steps (wav, stress, injection, velocity, step counter), the
-            # adjoint steps (two weight and two gather kernels, residual injection), zeroing of 8 gradients
-            "gpu_launches": args.steps * ((2 * p.nt - kept) * 5 + p.nt * (3 + 5) + nseg + 8),
+            # per gradient: forward and recompute steps (stress and velocity, which take recorder and injection along),
+            # the shell of every kept step, the adjoint steps (two kernels, residual injection), and per segment the
+            # first V, its rebuild or restore, the first bases and the fold of the sums
+            "gpu_launches": args.steps * ((2 * p.nt - kept) * 2 + kept + p.nt * 3 + nseg * 4),
             "clocks": clk.summary()}
     prob.close()
     if rank == 0 and not args.no_cpu_baseline:
@@ -1157,7 +1158,8 @@ def main():
                                 "d2h_bytes_per_step": d2h,
                                 "what": "the host-built medium from pinned memory (5 arrays; the 6 averaged ones "
                                         "formed on the device), then the same calls"},
-            "gpu_launches": args.steps * (3 + 1 + 1),
+            # stress (with recorder and injection) and velocity (with the step counter)
+            "gpu_launches": args.steps * 2,
             "clocks": clk.summary()}
     sim.close()
     if rank == 0 and args.accuracy:
