@@ -259,10 +259,8 @@ extern "C" int swpc_destroy(swpc_ctx *c) {
         if (c->gy[q]) cudaFree(c->gy[q]);
         if (c->gz[q]) cudaFree(c->gz[q]);
     }
-    for (InjColumns *ic : {&c->glut_cols, &c->bf_cols, &c->green_cols}) {
-        if (ic->list) cudaFree(ic->list);
-        if (ic->col) cudaFree(ic->col);
-    }
+    for (InjColumns *ic : {&c->glut_cols, &c->bf_cols, &c->green_cols})
+        if (ic->list) cudaFree(ic->list);   // owns the block of list and columns
     if (c->h_vmax) cudaFreeHost(c->h_vmax);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
@@ -830,8 +828,8 @@ static int build_list(swpc_ctx *c, std::vector<InjEntry> &v, InjEntry **dptr, in
 // update reaches, with FP16 stress arrays or 2D body forces (another density
 // cell) has none and keeps its own launch.
 static int build_columns(swpc_ctx *c, const std::vector<InjEntry> &v, InjColumns &ic) {
-    if (ic.list) { cudaFree(ic.list); ic.list = nullptr; }
-    if (ic.col) { cudaFree(ic.col); ic.col = nullptr; }
+    if (ic.list) cudaFree(ic.list);   // owns the block of both
+    ic = InjColumns();
     const Geo &g = c->g;
     std::vector<std::pair<int, int>> order;   // (column, list position): list order within a column
     for (size_t n = 0; n < v.size(); n++) {
@@ -857,10 +855,14 @@ static int build_columns(swpc_ctx *c, const std::vector<InjEntry> &v, InjColumns
         q.last = n + 1 == order.size() || order[n + 1].first != order[n].first;
         if (n == 0 || order[n - 1].first != order[n].first) col[order[n].first] = (int)n;
     }
-    RC(dalloc(c, &ic.list, list.size()));
-    RC(dalloc(c, &ic.col, col.size()));
-    CK(cudaMemcpyAsync(ic.list, list.data(), list.size() * sizeof(InjCell), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(ic.col, col.data(), col.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    // one block, the list first
+    const size_t nl = list.size() * sizeof(InjCell), nc = col.size() * sizeof(int);
+    char *blk = nullptr;
+    RC(dalloc(c, &blk, nl + nc));
+    ic.list = reinterpret_cast<InjCell *>(blk);
+    ic.col = reinterpret_cast<int *>(blk + nl);
+    CK(cudaMemcpyAsync(ic.list, list.data(), nl, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(ic.col, col.data(), nc, cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     return SWPC_OK;
 }
