@@ -142,6 +142,8 @@ struct GStrOps {
     }
     __device__ __forceinline__ float sown(int f) const { return ldS<PREC>(S[f], e, sc_sS_in(a.scale, f)); }
     __device__ __forceinline__ float r(int q) const { return ldR<PREC>(a.R[q] + so, e, sc_sR_in(a.scale)); }
+    __device__ __forceinline__ float iS(int f) const { return sc_iS(a.scale, f); }
+    __device__ __forceinline__ float iR() const { return sc_iR(a.scale); }
     // 0 mu, 1 lam, 2 taup, 3 taus, 4 muyz, 5 muxz, 6 muxy
     __device__ __forceinline__ float med(int m) const {
         const float *p = m == 0 ? a.mu : m == 1 ? a.lam : m == 2 ? a.taup : m == 3 ? a.taus
@@ -203,9 +205,9 @@ __device__ __forceinline__ void stress_interior(const Str3Args &a, const Ops &o,
     }
     const float taup_plus1 = 1 + taup1 * (1 + a.d2);
     const float taus_plus1 = 1 + taus1 * (1 + a.d2);
-    stS<PREC>(S[0], e, sxx + (lam2mu * taup_plus1 * d3v3 - mu2 * taus_plus1 * dyVy_dzVz + Rxx_n) * dt, sc_iS(a.scale, 0));
-    stS<PREC>(S[1], e, syy + (lam2mu * taup_plus1 * d3v3 - mu2 * taus_plus1 * dxVx_dzVz + Ryy_n) * dt, sc_iS(a.scale, 1));
-    stS<PREC>(S[2], e, szz + (lam2mu * taup_plus1 * d3v3 - mu2 * taus_plus1 * dxVx_dyVy + Rzz_n) * dt, sc_iS(a.scale, 2));
+    stS<PREC>(S[0], e, sxx + (lam2mu * taup_plus1 * d3v3 - mu2 * taus_plus1 * dyVy_dzVz + Rxx_n) * dt, o.iS(0));
+    stS<PREC>(S[1], e, syy + (lam2mu * taup_plus1 * d3v3 - mu2 * taus_plus1 * dxVx_dzVz + Ryy_n) * dt, o.iS(1));
+    stS<PREC>(S[2], e, szz + (lam2mu * taup_plus1 * d3v3 - mu2 * taus_plus1 * dxVx_dyVy + Rzz_n) * dt, o.iS(2));
 
     // shear components (m_kernel.f90:282-311)
     const float dxVy_dyVx = (vyip - vy0) * re40x - (vyip2 - vyim) * re41x
@@ -224,13 +226,14 @@ __device__ __forceinline__ void stress_interior(const Str3Args &a, const Ops &o,
         Rxz_n = Rxz_n + a.d1[m] * r[4][m];
         Rxy_n = Rxy_n + a.d1[m] * r[5][m];
     }
-    stS<PREC>(S[3], e, syz + (muyz * taus_plus1 * dyVz_dzVy + Ryz_n) * dt, sc_iS(a.scale, 3));
-    stS<PREC>(S[4], e, sxz + (muxz * taus_plus1 * dxVz_dzVx + Rxz_n) * dt, sc_iS(a.scale, 4));
-    stS<PREC>(S[5], e, sxy + (muxy * taus_plus1 * dxVy_dyVx + Rxy_n) * dt, sc_iS(a.scale, 5));
+    stS<PREC>(S[3], e, syz + (muyz * taus_plus1 * dyVz_dzVy + Ryz_n) * dt, o.iS(3));
+    stS<PREC>(S[4], e, sxz + (muxz * taus_plus1 * dxVz_dzVx + Rxz_n) * dt, o.iS(4));
+    stS<PREC>(S[5], e, sxy + (muxy * taus_plus1 * dxVy_dyVx + Rxy_n) * dt, o.iS(5));
+    const float iR = o.iR();
 #pragma unroll
     for (int c = 0; c < 6; c++)
 #pragma unroll
-        for (int m = 0; m < NM; m++) stR<PREC>(a.R[c * 3 + m] + so, e, r[c][m], sc_iR(a.scale, c * 3 + m));
+        for (int m = 0; m < NM; m++) stR<PREC>(a.R[c * 3 + m] + so, e, r[c][m], iR);
 }
 
 // absorb_p__update_vel (m_absorb_p.f90:248-309) for one absorber cell: the
@@ -357,9 +360,9 @@ __device__ __forceinline__ void stress_absorber(const Str3Args &a, const Ops &o,
     const float dxVx_ade = gxc.x * dxVx + gxc.y * vaxVx;
     const float dyVy_ade = gyc.x * dyVy + gyc.y * vayVy;
     const float dzVz_ade = gzc.x * dzVz + gzc.y * vazVz;
-    stS<PREC>(S[0], e, sxx + (lam2mu_R * dxVx_ade + lam_R * (dyVy_ade + dzVz_ade)) * dt, sc_iS(a.scale, 0));
-    stS<PREC>(S[1], e, syy + (lam2mu_R * dyVy_ade + lam_R * (dxVx_ade + dzVz_ade)) * dt, sc_iS(a.scale, 1));
-    stS<PREC>(S[2], e, szz + (lam2mu_R * dzVz_ade + lam_R * (dxVx_ade + dyVy_ade)) * dt, sc_iS(a.scale, 2));
+    stS<PREC>(S[0], e, sxx + (lam2mu_R * dxVx_ade + lam_R * (dyVy_ade + dzVz_ade)) * dt, o.iS(0));
+    stS<PREC>(S[1], e, syy + (lam2mu_R * dyVy_ade + lam_R * (dxVx_ade + dzVz_ade)) * dt, o.iS(1));
+    stS<PREC>(S[2], e, szz + (lam2mu_R * dzVz_ade + lam_R * (dxVx_ade + dyVy_ade)) * dt, o.iS(2));
     sts(&axVx[q], gxc.z * vaxVx + gxc.w * dxVx * dt);
     sts(&ayVy[q], gyc.z * vayVy + gyc.w * dyVy * dt);
     sts(&azVz[q], gzc.z * vazVz + gzc.w * dzVz * dt);
@@ -370,9 +373,9 @@ __device__ __forceinline__ void stress_absorber(const Str3Args &a, const Ops &o,
     const float dyVz = (vzjp - vz0) * r20y;
     const float dzVx = (vxkp - vx0) * r20z;
     const float dzVy = (vykp - vy0) * r20z;
-    stS<PREC>(S[3], e, syz + muyz * (gye.x * dyVz + gze.x * dzVy + gye.y * vayVz + gze.y * vazVy) * dt, sc_iS(a.scale, 3));
-    stS<PREC>(S[4], e, sxz + muxz * (gxe.x * dxVz + gze.x * dzVx + gxe.y * vaxVz + gze.y * vazVx) * dt, sc_iS(a.scale, 4));
-    stS<PREC>(S[5], e, sxy + muxy * (gxe.x * dxVy + gye.x * dyVx + gxe.y * vaxVy + gye.y * vayVx) * dt, sc_iS(a.scale, 5));
+    stS<PREC>(S[3], e, syz + muyz * (gye.x * dyVz + gze.x * dzVy + gye.y * vayVz + gze.y * vazVy) * dt, o.iS(3));
+    stS<PREC>(S[4], e, sxz + muxz * (gxe.x * dxVz + gze.x * dzVx + gxe.y * vaxVz + gze.y * vazVx) * dt, o.iS(4));
+    stS<PREC>(S[5], e, sxy + muxy * (gxe.x * dxVy + gye.x * dyVx + gxe.y * vaxVy + gye.y * vayVx) * dt, o.iS(5));
     sts(&ayVx[q], gye.z * vayVx + gye.w * dyVx * dt);
     sts(&azVx[q], gze.z * vazVx + gze.w * dzVx * dt);
     sts(&axVy[q], gxe.z * vaxVy + gxe.w * dxVy * dt);

@@ -89,24 +89,26 @@ struct SStrOps {
     const float *sv;   // member's V box
     const float *sm;   // medium box: lam mu taup taus muyz muxz muxy
     int tx, ty, tz;
-    const Str3Args &a;   // FP16 scales of S and R (PREC_F16_SR)
+    const float *sc;   // FP16 scales
     __device__ __forceinline__ int at(int f) const { return ((f * BJ + tz) * BI + ty) * KT + tx; }
     __device__ __forceinline__ float v(int c, int dk, int di, int dj) const {
         return sv[((c * (BJ + 4) + tz + 2 + dj) * (BI + 4) + ty + 2 + di) * KB + tx + 4 + dk];
     }
     __device__ __forceinline__ float sown(int f) const {
-        if constexpr (PREC == PREC_F16_SR) return __half2float(reinterpret_cast<const __half *>(ss)[at(f)]) * sc_sS_in(a.scale, f);
+        if constexpr (PREC == PREC_F16_SR) return __half2float(reinterpret_cast<const __half *>(ss)[at(f)]) * sc_sS_in(sc, f);
         else return ss[at(f)];
     }
     __device__ __forceinline__ float r(int q) const {
         const int f = (q / 3) * NM + q % 3;
-        if constexpr (PREC == PREC_F16_SR) return __half2float(reinterpret_cast<const __half *>(ss)[at(6 + f)]) * sc_sR_in(a.scale);
+        if constexpr (PREC == PREC_F16_SR) return __half2float(reinterpret_cast<const __half *>(ss)[at(6 + f)]) * sc_sR_in(sc);
         else if constexpr (PREC == PREC_BF16_R)
             return __bfloat162float(reinterpret_cast<const __nv_bfloat16 *>(ss + StrBoxes<NM, BI, BJ, 1, PREC>::oR)[at(f)]);
         else if constexpr (PREC == PREC_F16_R)
-            return __half2float(reinterpret_cast<const __half *>(ss + StrBoxes<NM, BI, BJ, 1, PREC>::oR)[at(f)]) * sc_sR_in(a.scale);
+            return __half2float(reinterpret_cast<const __half *>(ss + StrBoxes<NM, BI, BJ, 1, PREC>::oR)[at(f)]) * sc_sR_in(sc);
         else return ss[at(6 + f)];
     }
+    __device__ __forceinline__ float iS(int f) const { return sc_iS(sc, f); }
+    __device__ __forceinline__ float iR() const { return sc_iR(sc); }
     // 0 mu, 1 lam, 2 taup, 3 taus, 4 muyz, 5 muxz, 6 muxy
     __device__ __forceinline__ float med(int m) const { return sm[at(m == 0 ? 1 : m == 1 ? 0 : m)]; }
 };
@@ -133,6 +135,7 @@ __global__ void __launch_bounds__(KT * BI * BJ,
     extern __shared__ __align__(128) unsigned char smraw[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ unsigned long long limit;
+    __shared__ float sc[kScaleUsed];   // PREC_F16_SR: the scales (the two of PREC_F16_R stay in registers)
     float *sm = aligned128(smraw);
     const Geo g = a.g;
     if (blockIdx.x < x.nwav) {
@@ -195,14 +198,15 @@ __global__ void __launch_bounds__(KT * BI * BJ,
         for (int mm = 0; mm < (PRE ? M : 1); mm++)
             if (mm < T.nmem) xs[mm] = aux_load(a.aV, (long long)(T.m0 + mm) * t.ao, a.pmlcol, g, k, i, j);
     }
-    __syncthreads();   // barrier initialised, wait limit set
+    if (PREC == PREC_F16_SR && ty == 0 && tz == 0 && tx < kScaleUsed) sc[tx] = a.scale[tx];
+    __syncthreads();   // barrier initialised, wait limit and scales set
     if (!wait_tiles(&bar, t.err, limit) || !mine) return;   // the copy failed, or no cell of this launch here
 #pragma unroll
     for (int mm = 0; mm < M; mm++) {
         if (mm >= T.nmem) break;
         const long long so = (long long)(T.m0 + mm) * t.so, ao = (long long)(T.m0 + mm) * t.ao;
         const float *p = sm + L::oMem(mm);
-        const SStrOps<NM, BI, BJ, PREC> o{p, p + up32(L::nState), sm, tx, ty, tz, a};
+        const SStrOps<NM, BI, BJ, PREC> o{p, p + up32(L::nState), sm, tx, ty, tz, PREC == PREC_F16_SR ? sc : a.scale};
         float *const Sp[6] = {a.Sxx + so, a.Syy + so, a.Szz + so, a.Syz + so, a.Sxz + so, a.Sxy + so};
         if (interior) {
             stress_interior<NM, PREC>(a, o, sgn, Sp, e, so);
@@ -252,14 +256,14 @@ struct SVelOps {
     const float *mem;   // member's boxes
     const float *sb;    // bx by bz
     int tx, ty, jj;
-    const Vel3Args &a;  // FP16 scales of S (PREC_F16_SR)
+    const float *sS;    // FP16 scales of S (PREC_F16_SR)
     using L = VelBoxes<BI, BJ, 1, PREC>;
     __device__ __forceinline__ int at(int c) const { return ((c * BJ + jj) * BI + ty) * KT + tx; }
     __device__ __forceinline__ float v(int c) const { return mem[L::oV + at(c)]; }
     __device__ __forceinline__ float b(int c) const { return sb[at(c)]; }
     // element q of the box at float offset o
     __device__ __forceinline__ float el(int f, int o, int q) const {
-        if constexpr (L::H) return __half2float(reinterpret_cast<const __half *>(mem + o)[q]) * sc_sS(a.scale, f);
+        if constexpr (L::H) return __half2float(reinterpret_cast<const __half *>(mem + o)[q]) * sS[f];
         else return mem[o + q];
     }
     __device__ __forceinline__ float s(int f, int dk, int di, int dj) const {
@@ -292,6 +296,7 @@ __global__ void __launch_bounds__(KT * BI, (blocks_per_sm<VelBoxes<BI, BJ, M, PR
     extern __shared__ __align__(128) unsigned char smraw[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ unsigned long long limit;
+    __shared__ float sS[6];   // FP16 scales of S (PREC_F16_SR)
     float *sm = aligned128(smraw);
     const Geo g = a.g;
     const Tile T = tile_of<M>(t, BI, BJ, t.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
@@ -371,7 +376,8 @@ __global__ void __launch_bounds__(KT * BI, (blocks_per_sm<VelBoxes<BI, BJ, M, PR
                     xs[mm][jj] = aux_load(a.aS, (long long)(T.m0 + mm) * t.ao, a.pmlcol, g, k, i, j);
             }
     }
-    __syncthreads();   // barrier initialised, wait limit set
+    if (PREC == PREC_F16_SR && ty == 0 && tx < 6) sS[tx] = sc_sS(a.scale, tx);
+    __syncthreads();   // barrier initialised, wait limit and scales set
     if (!wait_tiles(&bar, t.err, limit) || !col_ok) return;   // the copy failed, or no cell of this launch here
 #pragma unroll
     for (int mm = 0; mm < M; mm++) {
@@ -382,7 +388,7 @@ __global__ void __launch_bounds__(KT * BI, (blocks_per_sm<VelBoxes<BI, BJ, M, PR
             const int j = T.j0 + jj;
             if (j > g.ny) break;
             const bool interior = i >= a.ibk && i <= a.iek && j >= a.jbk && j <= a.jek && k <= a.kek;
-            const SVelOps<BI, BJ, PREC> o{sm + L::oMem(mm), sm, tx, ty, jj, a};
+            const SVelOps<BI, BJ, PREC> o{sm + L::oMem(mm), sm, tx, ty, jj, sS};
             const long long e = col_index(g, i, j) * g.Kp + (k - 1 + KH);
             if (interior && (a.mask & 1)) {
                 vel_interior<PREC>(a, o, sgn[jj], a.Vx + so, a.Vy + so, a.Vz + so, e);

@@ -14,20 +14,25 @@ enum InjMode { INJ_GLUT = 0, INJ_GLUT4 = 1, INJ_GLUT2 = 2, INJ_BF3 = 3, INJ_GREE
 // for stress array f, stored = value * iS[f], and sR, iR for the memory
 // variables, which share one scale (FP16 keeps 11 significant bits over 29
 // binades, so arrays that differ by orders of magnitude lose nothing by
-// sharing it, and the stress kernel reads it from one read-only address).
+// sharing it, and the stress kernel reads it from one address).
 // Layout: [0..5] sS_in, [6] sR_in (what the stored values meant before this
 // step's stress update: only the stress kernel reads them), [7..12] sS,
 // [13..18] iS, [19] sR, [20] iR (what it writes, and what every other kernel
 // and transfer uses).  A re-centring changes the latter before the stress
 // update, which converts every value as it rewrites it; the former follow
 // after it.  FP32 storage keeps them 1.
-constexpr int kScaleFloats = 48;
-__device__ __forceinline__ float sc_sS_in(const float *s, int f) { return __ldg(s + f); }
-__device__ __forceinline__ float sc_sR_in(const float *s) { return __ldg(s + 6); }
-__device__ __forceinline__ float sc_sS(const float *s, int f) { return __ldg(s + 7 + f); }
-__device__ __forceinline__ float sc_iS(const float *s, int f) { return __ldg(s + 13 + f); }
-__device__ __forceinline__ float sc_sR(const float *s, int) { return __ldg(s + 19); }
-__device__ __forceinline__ float sc_iR(const float *s, int) { return __ldg(s + 20); }
+// The re-centring kernels write them between a step's launches, and a staged
+// launch may be resident before the kernel ahead of it has ended: the scales
+// are read by plain loads, after the launch's pdl_wait (a read-only load would
+// ask for data that nothing writes while the kernel is resident, and may be
+// moved ahead of the wait).
+constexpr int kScaleFloats = 48, kScaleUsed = 21;
+__device__ __forceinline__ float sc_sS_in(const float *s, int f) { return s[f]; }
+__device__ __forceinline__ float sc_sR_in(const float *s) { return s[6]; }
+__device__ __forceinline__ float sc_sS(const float *s, int f) { return s[7 + f]; }
+__device__ __forceinline__ float sc_iS(const float *s, int f) { return s[13 + f]; }
+__device__ __forceinline__ float sc_sR(const float *s) { return s[19]; }
+__device__ __forceinline__ float sc_iR(const float *s) { return s[20]; }
 
 // Point sources that a staged launch adds to the cells it updates
 // (swpc_step.cuh): col[column] = the column's first entry in list, -1 for none
