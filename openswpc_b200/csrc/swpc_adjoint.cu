@@ -1226,8 +1226,7 @@ int err(swpc_ctx *c, int code, const char *m) { return set_err(c, code, m); }
         if (_rc) return _rc;                                 \
     } while (0)
 
-static int adj_alloc(swpc_ctx *c) {
-    if (c->adj) return SWPC_OK;
+static int adj_build(swpc_ctx *c) {
     auto *s = new swpc_adj_state();
     c->adj = s;
     const long long n = c->g.ncell;
@@ -1305,6 +1304,20 @@ void adj_free(swpc_ctx *c) {
     c->adj = nullptr;
 }
 }  // namespace swpc
+
+// The adjoint state, complete or not there: a call that finds no room leaves
+// nothing behind, and the next one builds it anew.
+static int adj_alloc(swpc_ctx *c) {
+    if (c->adj) return SWPC_OK;
+    const long long bytes = c->bytes;
+    const int rc = adj_build(c);
+    if (rc) {
+        cudaStreamSynchronize(c->stream);   // the clears of the blocks to be freed
+        adj_free(c);
+        c->bytes = bytes;
+    }
+    return rc;
+}
 
 static int adj_ready(swpc_ctx *c) {
     if (!c) return SWPC_ERR_ARG;
@@ -1873,13 +1886,13 @@ extern "C" int swpc_gradient(swpc_ctx *c, const float *obs, int ckpt, double *mi
             return err(c, SWPC_ERR_NOMEM, "no room for the checkpoints and slots (raise ckpt, lower the slot "
                                           "memory or shrink the grid)");
         }
-        s->ckpt = ckpt; s->nseg = nseg; s->ck_floats = ckf; s->slot_cap = cap; s->ntail = ntail;
-        s->keep_floats = need_keep;
         // the staged stress phase reads the forward V of a slot with its halo
         Geo gs = c->g;
         gs.Kp = sg.Kp; gs.Ip = sg.Ip; gs.Jp = sg.Jp; gs.ncell = sg.n;
         if (!tma_encode_box(s->maps->v1, s->slots, gs, (long long)kSlotFields * cap, tma::KB, adjt::BI + 3, adjt::BJA + 3, 1))
             return err(c, SWPC_ERR_CUDA, "cuTensorMapEncodeTiled failed for the recompute slots");
+        s->ckpt = ckpt; s->nseg = nseg; s->ck_floats = ckf; s->slot_cap = cap; s->ntail = ntail;
+        s->keep_floats = need_keep;
     }
     if (ntail > 0 && keeps_shell(c) && s->nshell != nshell) {
         const std::vector<int> sh = shell_cells(c, sg);

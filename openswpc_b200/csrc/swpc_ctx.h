@@ -280,6 +280,7 @@ int dalloc(swpc_ctx *c, T **p, size_t n) {
     if (n == 0) n = 1;
     cudaError_t e = cudaMalloc((void **)p, n * sizeof(T));
     if (e != cudaSuccess) {
+        cudaGetLastError();   // the launches that follow do not report it again
         *p = nullptr;
         return set_err(c, SWPC_ERR_NOMEM, std::string("cudaMalloc failed: ") + cudaGetErrorString(e));
     }
