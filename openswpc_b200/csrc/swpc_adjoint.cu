@@ -69,6 +69,7 @@ struct swpc_adj_state {
     double *grad[8] = {};                // lam mu muyz muxz muxy bx by bz: FP64 totals
     float *gpart[8] = {};                // the same, FP32 partial sums of the current segment
     float *res = nullptr;                // receiver residuals (nst, 3, ntw)
+    size_t res_cap = 0;                  // floats allocated: the recorder may be set up again
     int ckpt = 0, nseg = 0;
     float *ckpool = nullptr;             // checkpoints: V S R aux per segment
     float *slots = nullptr;              // V and the stress divergences after each step of a segment, or of
@@ -1907,7 +1908,13 @@ extern "C" int swpc_gradient(swpc_ctx *c, const float *obs, int ckpt, double *mi
     auto kept_first = [&](int g) { return s->keep + (size_t)(g - gT) * kseg; };
     auto kept_step = [&](int it) { return s->keep + (size_t)ntail * kseg + (size_t)(it - itT0) * kstep; };
     const size_t nres = (size_t)c->nst * 3 * c->ntw;
-    if (!s->res) ACK(cudaMalloc((void **)&s->res, nres * sizeof(float)));
+    if (s->res_cap < nres) {
+        if (s->res) cudaFree(s->res);
+        s->res = nullptr;
+        s->res_cap = 0;
+        ACK(cudaMalloc((void **)&s->res, nres * sizeof(float)));
+        s->res_cap = nres;
+    }
     // 1. forward from rest with a checkpoint before every recomputed segment; the trailing segments keep their
     //    steps instead (the recorders run in both)
     rc = zero_state(c);

@@ -4,7 +4,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from openswpc_b200._lib import check, fptr
+from openswpc_b200._lib import WAV_V, check, fptr, iptr
 from openswpc_b200.swpc3d import Swpc3D
 from tests.models import small3d
 
@@ -53,3 +53,26 @@ def test_gradient_after_the_adjoint_state_found_no_room():
     _same(got, _gradient(fresh, p, obs))
     g.close()
     fresh.close()
+
+
+def test_gradient_after_the_recorder_was_set_up_again():
+    """A recorder set up again with more samples than the gradient before had:
+    misfit and gradients equal those of a fresh context with that recorder."""
+    p = small3d(nx=40, ny=36, nz=32, na=8, nt=24)
+    g = Swpc3D(p)
+    rng = np.random.default_rng(4)
+
+    def recorder(r, nst, ntdec_w):
+        q = np.random.default_rng(nst)
+        pos = [q.integers(p.na + 2, n - p.na - 2, nst).astype(np.int32) for n in (p.nx, p.ny, p.nz)]
+        check(r.ctx, r.lib.swpc_wav_setup(r.ctx, nst, *(iptr(a) for a in pos), ntdec_w, WAV_V, r.M0, r.UC))
+
+    for nst, ntdec_w in ((2, 8), (40, 8), (40, 1), (2, 8)):
+        obs = rng.standard_normal((nst, 3, (p.nt - 1) // ntdec_w + 1)).astype(np.float32)
+        recorder(g, nst, ntdec_w)
+        got = _gradient(g, p, obs)
+        fresh = Swpc3D(p)
+        recorder(fresh, nst, ntdec_w)
+        _same(got, _gradient(fresh, p, obs))
+        fresh.close()
+    g.close()
