@@ -184,15 +184,18 @@ class Misfit3D:
         host but the traces and the misfit)."""
         s, p = self.solver, self.p
         on_dev = self._on_device(vp, vs, rho)
+        if on_dev:
+            vp, vs, rho = (self._dev(t) for t in (vp, vs, rho))   # once, for the model and for its gradient
         self._set_model(vp, vs, rho)
         J = C.c_double()
         check(s.ctx, s.lib.swpc_gradient(s.ctx, fptr(self.obs), self.ckpt, C.byref(J)))
         shape = (p.ny + 6, p.nx + 6, p.nz + 6)
         if on_dev:
-            m = [self._dev(t) for t in (vp, vs, rho)]
-            out = [torch.empty(shape, dtype=torch.float64, device=m[0].device) for _ in range(3)]
+            out = [torch.empty(shape, dtype=torch.float64, device=vp.device) for _ in range(3)]
             ptr = lambda t: C.c_void_p(t.data_ptr())
-            check(s.ctx, s.lib.swpc_gradient_model_device(s.ctx, ptr(m[0]), ptr(m[1]), ptr(m[2]), p.nz + 6,
+            # the library's stream reads the model and writes out at once: torch's work on their memory is done
+            torch.cuda.current_stream(vp.device).synchronize()
+            check(s.ctx, s.lib.swpc_gradient_model_device(s.ctx, ptr(vp), ptr(vs), ptr(rho), p.nz + 6,
                                                           p.nx + 6, ptr(out[0]), ptr(out[1]), ptr(out[2])))
             return J.value, out[0], out[1], out[2]
         f = lambda a: np.ascontiguousarray(a, np.float32).reshape(shape)

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from openswpc_b200._lib import WAV_V, check, fptr, iptr
+from openswpc_b200.params import Station
 from openswpc_b200.swpc3d import Swpc3D
 from tests.models import small3d
 
@@ -76,3 +77,28 @@ def test_gradient_after_the_recorder_was_set_up_again():
         _same(got, _gradient(fresh, p, obs))
         fresh.close()
     g.close()
+
+
+def test_device_gradient_of_converted_models():
+    """float64 and transposed CUDA models, which torch converts on its own
+    stream before the library reads them, give the bits of contiguous float32
+    ones (256 x 256 x 128 cells: the conversion outlasts the host's way to
+    the kernel)."""
+    import torch
+    from openswpc_b200.adjoint import Misfit3D
+    p = small3d(nx=256, ny=256, nz=128, na=12, nt=12, stations=[Station(1.0, 0.5, 6.0, "st", "dep")])
+    shape = (p.ny + 6, p.nx + 6, p.nz + 6)
+    q = np.full(shape, 200.0, np.float32)
+    vs = np.full(shape, 3.0, np.float32)
+    vs *= 1 + 0.05 * np.random.default_rng(2).random(shape, np.float32)
+    vp, rho = vs * np.float32(1.75), np.full(shape, 2.7, np.float32)
+    prob = Misfit3D(p, vp, vs, rho, q, q, np.ones((1, 3, p.nt), np.float32), ckpt=4)
+    f32 = [torch.from_numpy(a).cuda() for a in (vp, vs, rho)]
+    ref = prob.gradient(*f32)
+    assert all(float(g.abs().max()) > 0 for g in ref[1:])
+    for model in ([t.double() for t in f32], [t.permute(2, 1, 0).contiguous().permute(2, 1, 0) for t in f32]):
+        got = prob.gradient(*model)
+        assert got[0] == ref[0]
+        for a, b in zip(got[1:], ref[1:]):
+            assert torch.equal(a.view(torch.int64), b.view(torch.int64))
+    prob.close()
