@@ -197,7 +197,10 @@ int swpc_vmodel_upload(swpc_ctx *ctx, const float *rho, const float *lam, const 
  * over the memory box (leading extents ld_k, ld_i), the moduli formed on the
  * device as vmodel_lhm forms them (m_vmodel_lhm.f90:146-148, mu = rho vs vs,
  * lam = rho (vp vp - 2 vs vs)); bitwise swpc_vmodel_upload of the moduli a
- * host computes in that order.  For models that already live on the GPU. */
+ * host computes in that order.  For models that already live on the GPU.
+ * Device arrays that a caller hands over (here, xi above, the gradient of
+ * swpc_gradient_model_device) are read and written on the context's stream
+ * at once: the caller's own work on them must have completed. */
 int swpc_vmodel_velocity_device(swpc_ctx *ctx, const float *vp, const float *vs, const float *rho, const float *qp,
                                 const float *qs, int ld_k, int ld_i);
 int swpc_medium_setup_device(swpc_ctx *ctx, float fq_min, float fq_max, float fq_ref, float *ts, float *scal,

@@ -278,6 +278,7 @@ class DeviceMedium:
                 import torch
 
                 assert tuple(xi.shape) == shape and xi.dtype == torch.float32 and xi.is_contiguous()
+                torch.cuda.current_stream(xi.device).synchronize()   # the library reads xi on its own stream
                 xp = C.cast(C.c_void_p(xi.data_ptr()), _lib._FP)
             else:
                 xi = np.ascontiguousarray(xi, np.float32)

@@ -1,5 +1,6 @@
-"""Order of torch's stream and the library's in the device gradient, on the
-CPU: a fake library that refuses arrays whose conversion nobody waited for."""
+"""Order of torch's stream and the library's where arrays on the device change
+hands, on the CPU: a fake library that refuses arrays whose conversion nobody
+waited for."""
 import types
 
 import numpy as np
@@ -53,3 +54,26 @@ def test_library_reads_converted_models_after_a_wait(form, monkeypatch):
         model = [torch.ones(shape[::-1]).permute(2, 1, 0) for _ in range(3)]
     prob.gradient(*model)
     assert calls[0] == "swpc_vmodel_velocity_device" and calls[-1] == "swpc_gradient_model_device"
+
+
+def test_library_reads_the_perturbation_after_a_wait(monkeypatch):
+    """A CUDA perturbation xi, which torch may still be writing on its stream,
+    is waited for before the medium set-up reads it."""
+    from openswpc_b200.swpc3d import DeviceMedium
+    p = small3d(nx=20, ny=18, nz=12, na=4, nt=4)
+    waited, calls = [], []
+
+    class Lib:
+        def __getattr__(self, name):
+            def call(*args):
+                assert waited, name
+                calls.append(name)
+                return 0
+            return call
+
+    xi = types.SimpleNamespace(shape=(p.ny + 6, p.nx + 6, p.nz + 6), dtype=torch.float32, is_cuda=True, device="cuda:0",
+                               data_ptr=lambda: 256, is_contiguous=lambda: True)
+    monkeypatch.setattr(torch.cuda, "current_stream",
+                        lambda d=None: types.SimpleNamespace(synchronize=lambda: waited.append(d)))
+    DeviceMedium(Lib(), None, p, xi)
+    assert calls[0] == "swpc_vmodel_lhm_device_opt" and waited == ["cuda:0"]
