@@ -1550,14 +1550,22 @@ static int build_graph(swpc_ctx *c, int steps, cudaGraphExec_t *exec) {
 constexpr int kGraphSteps = 10;
 constexpr long long kGraphManyCells = 1LL << 20;
 
+// the graphs of a run of nsteps steps, which replays `many` ten-step ones and `rest` single steps
+static int run_graphs(swpc_ctx *c, int nsteps, int *many, int *rest) {
+    *many = c->g.ncell <= kGraphManyCells ? nsteps / kGraphSteps : 0;
+    *rest = nsteps - *many * kGraphSteps;
+    if (*many) RC(build_graph(c, kGraphSteps, &c->graph_many));
+    if (*rest) RC(build_graph(c, 1, &c->graph_exec));
+    return SWPC_OK;
+}
+
 extern "C" int swpc_run(swpc_ctx *c, int it0, int nsteps) {
     if (!c) return SWPC_ERR_ARG;
     if (nsteps <= 0) return SWPC_OK;
     if (it0 < 1 || it0 + nsteps - 1 > c->d.nt) return set_err(c, SWPC_ERR_ARG, "time steps outside 1..nt");
     CK(cudaSetDevice(c->device));
-    const int many = c->g.ncell <= kGraphManyCells ? nsteps / kGraphSteps : 0, rest = nsteps - many * kGraphSteps;
-    if (many) RC(build_graph(c, kGraphSteps, &c->graph_many));
-    if (rest) RC(build_graph(c, 1, &c->graph_exec));
+    int many, rest;
+    RC(run_graphs(c, nsteps, &many, &rest));
     CK(cudaMemcpyAsync(c->d_it, &it0, sizeof(int), cudaMemcpyHostToDevice, c->stream));
     for (int n = 0; n < many; n++) CK(cudaGraphLaunch(c->graph_many, c->stream));
     for (int n = 0; n < rest; n++) CK(cudaGraphLaunch(c->graph_exec, c->stream));
@@ -1567,7 +1575,12 @@ extern "C" int swpc_run(swpc_ctx *c, int it0, int nsteps) {
 extern "C" int swpc_time_steps(swpc_ctx *c, int it0, int nsteps, float *ms) {
     if (!c || !ms) return SWPC_ERR_ARG;
     CK(cudaSetDevice(c->device));
-    RC(build_graph(c, 1, &c->graph_exec));
+    RC(check_ready(c));
+    // every graph of the run is there, on the device too, before the clock starts
+    int many = 0, rest = 0;
+    if (nsteps > 0) RC(run_graphs(c, nsteps, &many, &rest));
+    if (many) CK(cudaGraphUpload(c->graph_many, c->stream));
+    if (rest) CK(cudaGraphUpload(c->graph_exec, c->stream));
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
