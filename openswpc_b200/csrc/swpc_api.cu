@@ -831,7 +831,7 @@ static int build_columns(swpc_ctx *c, const std::vector<InjEntry> &v, InjColumns
     if (ic.list) cudaFree(ic.list);   // owns the block of both
     ic = InjColumns();
     const Geo &g = c->g;
-    std::vector<std::pair<int, int>> order;   // (column, list position): list order within a column
+    std::vector<std::pair<long long, int>> order;   // (cell, list position): by column, cell, list order
     for (size_t n = 0; n < v.size(); n++) {
         const InjEntry &e = v[n];
         const int col = (int)(e.cell / g.Kp), k = (int)(e.cell % g.Kp) - KH + 1;
@@ -839,21 +839,24 @@ static int build_columns(swpc_ctx *c, const std::vector<InjEntry> &v, InjColumns
         const bool half = c->prec == SWPC_PREC_F16_SR && e.field >= SWPC_F_SXX;
         if (k < 1 || k > g.nz || i < 1 || i > g.nx || (is3d(c) && (j < 1 || j > g.ny)) || half || e.mode > INJ_GREEN)
             return SWPC_OK;
-        order.push_back({col, (int)n});
+        order.push_back({e.cell, (int)n});
     }
     if (order.empty()) return SWPC_OK;
     std::sort(order.begin(), order.end());
     std::vector<InjCell> list(order.size());
     std::vector<int> col((size_t)g.Ip * g.Jp, -1);
-    for (size_t n = 0; n < order.size(); n++) {
+    int next = -1;   // column of the entry after this one
+    for (size_t n = order.size(); n-- > 0;) {
         const InjEntry &e = v[order[n].second];
+        const int cc = (int)(e.cell / g.Kp);
         InjCell &q = list[n];
         q.cell = e.cell;
         q.p = (e.field < SWPC_F_SXX ? c->V[e.field - SWPC_F_VX] : c->S[e.field - SWPC_F_SXX]) + e.cell;
         q.b = e.mode >= INJ_BF3 ? c->med[5 + e.bfield] + e.cell : nullptr;
         q.coef = e.coef; q.src = e.src; q.mode = e.mode;
-        q.last = n + 1 == order.size() || order[n + 1].first != order[n].first;
-        if (n == 0 || order[n - 1].first != order[n].first) col[order[n].first] = (int)n;
+        q.rest = cc == next ? list[n + 1].rest + 1 : 1;
+        col[cc] = (int)n;   // ends at the column's first entry
+        next = cc;
     }
     // one block, the list first
     const size_t nl = list.size() * sizeof(InjCell), nc = col.size() * sizeof(int);

@@ -51,13 +51,14 @@ struct InjEntry {
 };
 
 // An entry of the same lists as a staged update launch applies it: the
-// entries of one column stand together in list order, the last one marked.
+// entries of one column stand together, by cell and within a cell in list order.
 struct InjCell {
     long long cell;
     float *p;         // the value at the cell
     const float *b;   // the buoyancy there (body forces)
     float coef;
-    int src, mode, last;
+    int src, mode;
+    int rest;         // entries of the column from this one on
 };
 // One injection list by column (both null: the list has no such form).
 struct InjColumns {

@@ -127,3 +127,57 @@ def test_setup_between_runs(what):
         r.close()
     for a, b in zip(*out):
         assert np.abs(b).max() > 0 and _same(a, b)
+
+
+def _column(p, ks, i, j=None):
+    """One source per entry of ks, all in the column (i, j)."""
+    out = []
+    for n, k in enumerate(ks):
+        m = np.random.default_rng(n).uniform(-1, 1, 6)
+        y = p.ybeg + (j - 0.5) * p.dy if j else 0.0
+        out.append(Source(p.xbeg + (i - 0.5) * p.dx, y, p.zbeg + (k - 0.5) * p.dz, 0.0, 0.3, mo=1e15, mxx=m[0],
+                          myy=m[1], mzz=m[2], myz=m[3], mxz=m[4], mxy=m[5]))
+    return out
+
+
+# a fault from bottom to top, one whose subfaults share cells, and one with a cell of many sources between single ones
+@pytest.mark.parametrize("ks", [list(range(90, 6, -3)), list(range(8, 60)) * 2, [70, 9] + [30] * 9 + [31, 12]])
+def test_long_source_columns(ks):
+    """Columns with many sources, in any order of depth, give the bits of the
+    injection launch."""
+    p = small3d(nx=33, ny=29, nz=96, na=4, nt=12)
+    p.sources = _column(p, ks, 17, 15)
+    q = small2d("psv", nx=64, nz=96, na=4, nt=12)
+    q.sources = _column(q, ks, 30)
+    out = []
+    for flat in (False, True):
+        r, s = Swpc3D(p, medium_on_device=True), Swpc2D(q, "psv")
+        if flat:
+            for g, a, b in ((r, (2, 2, 1), (4, 2, 2)), (s, (1, 1, 1), (1, 1, 1))):
+                check(g.ctx, g.lib.swpc_set_launch(g.ctx, 0, *a))
+                check(g.ctx, g.lib.swpc_set_launch(g.ctx, 1, *b))
+        r.run(1, p.nt)
+        s.run(1, q.nt)
+        out.append([r.waveforms(), s.waveforms()] + [r.download(f) for f in range(9)] +
+                   [s.download(f) for f in s.field_ids.values()])
+        r.close()
+        s.close()
+    assert np.abs(out[0][2]).max() > 0
+    for a, b in zip(*out):
+        assert _same(a, b)
+
+
+def test_a_long_source_column_does_not_hold_the_step_back():
+    """Forty subfaults in one column cost no more than the same forty spread
+    over the grid, to a quarter of the step (walking the column's entries one
+    after another took the whole step again)."""
+    p = small3d(nx=96, ny=96, nz=160, na=8, nt=400)
+    spread = [s for n in range(40) for s in _column(p, [10 + 3 * n], 20 + 7 * n % 56, 20 + 11 * n % 56)]
+    best = []
+    for sources in (spread, _column(p, [10 + 3 * n for n in range(40)], 30, 30)):
+        p.sources = sources
+        r = Swpc3D(p, medium_on_device=True)
+        r.run(1, 40)
+        best.append(min(r.time_steps(41 + 40 * n, 40) for n in range(7)))
+        r.close()
+    assert best[1] <= 1.25 * best[0], best
