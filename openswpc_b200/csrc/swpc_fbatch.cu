@@ -25,6 +25,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <string>
 #include <vector>
 
@@ -568,33 +569,33 @@ extern "C" int swpc_fbatch_autotune(swpc_fbatch *b, int it0, int reps, int *step
     int it = it0;
     const int nt = b->c->d.nt;
     if (b->staged) {
-        // staged kernels: members per CTA and tile of the stress kernel, then of the velocity kernel
-        // launch order with the current shapes, then the shapes
-        {
-            int best = 0;
-            float best_ms = 1e30f;
-            for (int q = 0; q < 2 && it + 2 * reps - 1 <= nt; q++) {
-                FRC(swpc_fbatch_set_launch(b, 7, q, 0, 0));
-                float ms = 0.f;
-                FRC(fb_time(b, &it, reps, &ms));
-                if (ms < best_ms) { best_ms = ms; best = q; }
-            }
-            FRC(swpc_fbatch_set_launch(b, 7, best, 0, 0));
+        // launch order with the current shapes, then members per CTA and tile of the stress kernel, then of the
+        // velocity kernel; what is in use stays unless a candidate is faster
+        float best_ms = 1e30f;
+        int order = b->tiles_first;
+        for (int q = 0; q < 2 && it + 2 * reps - 1 <= nt; q++) {
+            FRC(swpc_fbatch_set_launch(b, 7, q, 0, 0));
+            float ms = 0.f;
+            FRC(fb_time(b, &it, reps, &ms));
+            if (ms < best_ms) { best_ms = ms; order = q; }
         }
-        const int sc[][3] = {{4, 2, 2}, {4, 4, 1}, {2, 4, 2}, {2, 2, 2}, {2, 2, 4}, {4, 1, 4}};
-        const int vc[][3] = {{4, 2, 2}, {4, 4, 1}, {4, 2, 1}, {2, 2, 2}, {2, 2, 4}, {4, 1, 4}};
+        FRC(swpc_fbatch_set_launch(b, 7, order, 0, 0));
+        using Shape = std::array<int, 3>;   // bi, bj, members per CTA
+        const std::vector<Shape> cand[2] = {
+            {{4, 2, 1}, {4, 2, 2}, {4, 4, 1}, {2, 4, 2}, {2, 2, 2}, {2, 2, 4}, {4, 1, 4}},
+            {{4, 2, 2}, {4, 4, 1}, {4, 2, 1}, {2, 2, 2}, {2, 2, 4}, {4, 1, 4}}};
         for (int kernel = 5; kernel <= 6; kernel++) {
-            const int(*cand)[3] = kernel == 5 ? sc : vc;
-            int best = 0;
-            float best_ms = 1e30f;
-            for (int q = 0; q < 6; q++) {
+            const Shape cur = kernel == 5 ? Shape{b->sbi, b->sbj, b->smpc} : Shape{b->vbi, b->vbj, b->vmpc};
+            Shape best = cur;
+            for (const Shape &s : cand[kernel - 5]) {
+                if (s == cur) continue;   // timed already
                 if (it + 2 * reps - 1 > nt) break;
-                FRC(swpc_fbatch_set_launch(b, kernel, cand[q][2], cand[q][0], cand[q][1]));
+                FRC(swpc_fbatch_set_launch(b, kernel, s[2], s[0], s[1]));
                 float ms = 0.f;
                 FRC(fb_time(b, &it, reps, &ms));
-                if (ms < best_ms) { best_ms = ms; best = q; }
+                if (ms < best_ms) { best_ms = ms; best = s; }
             }
-            FRC(swpc_fbatch_set_launch(b, kernel, cand[best][2], cand[best][0], cand[best][1]));
+            FRC(swpc_fbatch_set_launch(b, kernel, best[2], best[0], best[1]));
         }
         if (strip_out) *strip_out = 0;
     } else {

@@ -104,3 +104,29 @@ def test_autotune_keeps_results_and_bad_member_is_rejected():
         _lib.check(base.ctx, fb.lib.swpc_fbatch_green_source(fb.b, 2, 10, 10, 5, b"z", 0.0, 1.0, 0))
     fb.close()
     base.close()
+
+
+def test_autotune_keeps_the_launch_in_use_unless_another_is_faster():
+    """Without steps to spare nothing changes; with them the tuned form is no
+    slower than the one it started from (the default of a small batch is one
+    of the forms it may keep)."""
+    p = green_params(nt=700)
+    base = Swpc3D(p)
+    base.record(p.stations)
+    fb = ForceBatch3D(base, [(p.stations[s], c) for s, c in FORCES])
+    default = fb.launch()
+    used, _ = fb.autotune(p.nt, reps=2)
+    assert used == 0 and fb.launch() == default
+    fb.set_launch(5, 1, 2, 4)   # a shape that is no candidate
+    other = fb.launch()
+    used, _ = fb.autotune(p.nt, reps=2)
+    assert used == 0 and fb.launch() == other
+    bi, bj, mpc = default["stress"]
+    fb.set_launch(5, mpc, bi, bj)
+    fb.run(1, 40)
+    before = min(fb.time_steps(41 + 20 * n, 20) for n in range(5))
+    used, _ = fb.autotune(141, reps=8)
+    after = min(fb.time_steps(141 + used + 20 * n, 20) for n in range(5))
+    assert after <= 1.1 * before, (before, after, default, fb.launch())
+    fb.close()
+    base.close()
