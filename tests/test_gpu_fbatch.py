@@ -130,3 +130,9 @@ def test_autotune_keeps_the_launch_in_use_unless_another_is_faster():
     assert after <= 1.1 * before, (before, after, default, fb.launch())
     fb.close()
     base.close()
+
+
+@pytest.mark.parametrize("launch", [("staged", (4, 2, 1, 4, 2, 1, 1)), ("staged", (4, 4, 1, 4, 4, 1, 1))])
+def test_default_forms_equal_single_green_runs(launch):
+    """The forms a batch starts with below and above 6,000 tiles."""
+    test_members_equal_single_green_runs(launch)

@@ -181,3 +181,31 @@ def test_a_long_source_column_does_not_hold_the_step_back():
         best.append(min(r.time_steps(41 + 40 * n, 40) for n in range(7)))
         r.close()
     assert best[1] <= 1.25 * best[0], best
+
+
+# every staged tile a single FP32 run takes by default (four planes on larger grids, two on small ones), and mixed
+@pytest.mark.parametrize("nm", [3, 2, 1, 0])
+@pytest.mark.parametrize("mode", ["glut", "force", "green"])
+@pytest.mark.parametrize("sbj,vbj", [(4, 4), (2, 2), (4, 2)])
+def test_staged_tiles_against_the_flat_kernels(sbj, vbj, mode, nm):
+    """Stress and velocity tiles of four and of two planes, with the sources
+    inside the launches and any number of memory variables, give the bits of
+    the one-cell kernels; tiles partial in k, i and j."""
+    p = small3d(nx=42, ny=39, nz=45, na=6, nt=14, nm=nm, sw_wav_u=True, bf_mode=mode == "force",
+                green_mode=mode == "green", green_trise=0.3)
+    p.sources = _sources(p, 30, 11, 1.0)
+    out = []
+    for flat in (False, True):
+        r = Swpc3D(p, medium_on_device=True)
+        if mode == "green":
+            r.record(what=_lib.WAV_V | _lib.WAV_U)
+        for kernel, bj in ((0, 1), (1, 1)) if flat else ((5, sbj), (6, vbj)):
+            check(r.ctx, r.lib.swpc_set_launch(r.ctx, kernel, *((2, 2, 1) if flat else (1, 4, bj))))
+        r.run(1, p.nt)
+        out.append([r.waveforms(w) for w in (_lib.WAV_V, _lib.WAV_U)] + [r.download(f) for f in range(9)] +
+                   [r.download(_lib.F_R + 3 * c + m) for c in range(6) for m in range(nm)] +
+                   [r.download(_lib.F_AUX + q) for q in range(18)])
+        r.close()
+    assert np.abs(out[0][2]).max() > 0
+    for a, b in zip(*out):
+        assert _same(a, b)
