@@ -67,13 +67,19 @@ __device__ __forceinline__ const CUtensorMap *set_maps(const MapSet2D &s) {
     return reinterpret_cast<const CUtensorMap *>(&s);
 }
 
-// Resident CTAs the 8-thread P-SV kernels are compiled for, stress and velocity
-// (0: the compiler's choice of 54 and 44 registers): with 4 and 5, 64 and 48
-// registers, a 256 x 128 model takes 8.0 instead of 9.2 us a step, 1024 x 512
-// 16.8 instead of 18.3, 24 uneven models 190 instead of 197; SH kernels lose 5 %.
+// Resident CTAs the P-SV kernels are compiled for (0: the compiler's choice of
+// registers).  8 threads along i: stress 4 and velocity 5, 64 and 48 registers
+// instead of 54 and 44 (a 256 x 128 model 8.2 instead of 9.2 us a step, 1024 x
+// 512 16.4 instead of 17.7, 24 uneven models 184 instead of 192, 64 larger ones
+// 1455 instead of 1483); 4 threads: stress 8, 64 instead of 56 registers (those
+// 64 models 1404 instead of 1432).  SH kernels lose 5 % by it.
 template <int KIND, int TI>
-constexpr int min_ctas(int n) {
-    return KIND == 0 && TI == 8 ? n : 0;
+constexpr int stress_ctas() {
+    return KIND != 0 ? 0 : TI == 8 ? 4 : TI == 4 ? 8 : 0;
+}
+template <int KIND, int TI>
+constexpr int vel_ctas() {
+    return KIND == 0 && TI == 8 ? 5 : 0;
 }
 
 // the block's copy of the model descriptor
@@ -85,12 +91,12 @@ __device__ __forceinline__ void copy_model(const Model2D *__restrict__ models, i
 }
 
 // A batch's CTA copies its model's descriptor to shared memory; a single run
-// reads the parameter (no loads, and the band signs wait for no barrier).
-template <int G>
-__device__ __forceinline__ const Model2D &model_in(const MapGroup<G> &pm, const Model2D &copy) {
-    if constexpr (G > 1) return copy;
-    else return pm.model;
-}
+// reads the parameter (no loads, and the band signs wait for no barrier).  The
+// kernels take the address of their shared array themselves: handed through a
+// function with the parameter's it became a generic one, and 64 uneven P-SV
+// models took 1446 instead of 1372 us a step (8 and 4 threads along i), 24
+// smaller ones 188 instead of 182, 24 SH models 123 instead of 119.
+__device__ __forceinline__ const Model2D *model_of(const MapGroup<1> &pm) { return &pm.model; }
 
 // ---------------------------------------------------------------------------
 // shared-memory layouts (floats) and operand sources
@@ -172,7 +178,7 @@ __device__ __noinline__ void record(const Step2D &x, int cta) {
 }
 
 template <int KIND, int NM, int TI, int G>
-__global__ void __launch_bounds__(32 * TI, min_ctas<KIND, TI>(4)) stress2d_tma_kernel(const __grid_constant__ MapGroup<G> pm, int model0,
+__global__ void __launch_bounds__(32 * TI, stress_ctas<KIND, TI>()) stress2d_tma_kernel(const __grid_constant__ MapGroup<G> pm, int model0,
                                                                const Model2D *__restrict__ models,
                                                                const Tile2D *__restrict__ tiles, int mask,
                                                                Fields2D f, int *err,
@@ -215,7 +221,10 @@ __global__ void __launch_bounds__(32 * TI, min_ctas<KIND, TI>(4)) stress2d_tma_k
     pdl_wait();
     pdl_launch();
     __syncthreads();   // barrier initialised, wait limit and model descriptor set
-    const Model2D &M = model_in(pm, sM);
+    const Model2D *Mp;
+    if constexpr (G > 1) Mp = &sM;
+    else Mp = model_of(pm);
+    const Model2D &M = *Mp;
     // the band signs and source columns of this thread's cells are read while the tiles travel
     const int *icol = x.inj ? x.inj[tl.model].col : nullptr;
     int sg[RI], src[RI];
@@ -248,7 +257,7 @@ __global__ void __launch_bounds__(32 * TI, min_ctas<KIND, TI>(4)) stress2d_tma_k
 }
 
 template <int KIND, int TI, int G>
-__global__ void __launch_bounds__(32 * TI, min_ctas<KIND, TI>(5)) vel2d_tma_kernel(const __grid_constant__ MapGroup<G> pm, int model0,
+__global__ void __launch_bounds__(32 * TI, vel_ctas<KIND, TI>()) vel2d_tma_kernel(const __grid_constant__ MapGroup<G> pm, int model0,
                                                             const Model2D *__restrict__ models,
                                                             const Tile2D *__restrict__ tiles, int mask, Fields2D f,
                                                             int *err, int *it_next) {
@@ -292,7 +301,10 @@ __global__ void __launch_bounds__(32 * TI, min_ctas<KIND, TI>(5)) vel2d_tma_kern
     pdl_wait();
     pdl_launch();
     __syncthreads();   // barrier initialised, wait limit and model descriptor set
-    const Model2D &M = model_in(pm, sM);
+    const Model2D *Mp;
+    if constexpr (G > 1) Mp = &sM;
+    else Mp = model_of(pm);
+    const Model2D &M = *Mp;
     // the band signs of this thread's cells are read while the tiles travel
     int sg[RI];
 #pragma unroll
