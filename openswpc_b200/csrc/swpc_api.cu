@@ -425,6 +425,15 @@ static int stage_room(swpc_ctx *c, long long n) {
     return SWPC_OK;
 }
 
+static bool page_locked(const void *p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeHost;
+}
+
 int copy_box(swpc_ctx *c, float *dev, const float *host_in, float *host_out, int ld_k, int ld_i) {
     const Geo &g = c->g;
     const int nkb = g.nz + 6;             // k = -2 .. nz+3
@@ -435,13 +444,18 @@ int copy_box(swpc_ctx *c, float *dev, const float *host_in, float *host_out, int
     const long long plane = (long long)ld_i * ld_k;   // floats of a host plane
     // An upload of 256 KB or more, and a download into a box without padding
     // (a padded one keeps the elements between its rows): contiguous chunks of
-    // host planes (at most 16 MB) through a staging buffer, each repacked by a
-    // kernel.  The copy engine moves short rows at another pitch several times
-    // slower: a download of 107 x 93 x 67 cells takes 1.77 ms less than row by
-    // row, one of 46 x 42 x 38 cells 0.21 ms less.
+    // host planes (at most 16 Mi floats, 64 MiB, unless one plane is larger)
+    // through a staging buffer, each repacked by a kernel.  The copy engine
+    // moves short rows at another pitch several times slower: a download of 107
+    // x 93 x 67 cells takes 1.77 ms less than row by row, one of 46 x 42 x 38
+    // cells 0.21 ms less.  Into page-locked memory it is faster with a 2D model
+    // (2048 x 1024 166 us, packed 173; 517 x 259 26 and 33), and with rows from
+    // 512 bytes in boxes below 12 MB (102 x 86 x 261 cells 183 and 193 us; but
+    // 102 x 86 x 67 cells 76 and 65, 262 x 262 x 134 715 and 691).
     const int nj = (int)std::max<long long>(1, std::min<long long>(njb, (16LL << 20) / plane));
     const bool tight = ld_k == nkb && ld_i == nib;
-    bool staged = host_in ? plane * njb >= (1LL << 16) : tight;
+    bool staged = host_in ? plane * njb >= (1LL << 16)
+                          : tight && !(page_locked(host_out) && (!is3d(c) || (nkb >= 128 && plane * njb < (3LL << 20))));
     if (staged) {
         const int rc = stage_room(c, plane * nj);
         if (rc && host_in) return rc;

@@ -38,3 +38,20 @@ def test_download_box(kind, dims):
     assert np.all(pad[..., -3:] == -7.0)
     assert np.all(pad[..., -2:, :] == -7.0)
     run.close()
+
+
+# page-locked boxes on both sides of the row length and of the size at which a 3D download is packed, and 2D ones
+@pytest.mark.parametrize("kind,dims", [("3d", (250, 109, 101)), ("3d", (250, 102, 101)), ("3d", (121, 27, 25)),
+                                       ("3d", (122, 27, 25)), ("3d", (29, 31, 26)), ("psv", (33, 57, 1)),
+                                       ("sh", (250, 519, 1))])
+def test_download_into_page_locked_memory(kind, dims):
+    import torch
+    run = _run(kind, dims)
+    shape = ((dims[2] + 6,) if kind == "3d" else ()) + (dims[1] + 6, dims[0] + 6)
+    field = _lib.F_VY if kind == "sh" else _lib.F_VX
+    a = np.random.default_rng(4).standard_normal(shape).astype(np.float32)
+    run.upload(field, a)
+    b = torch.full(shape, -7.0).pin_memory().numpy()
+    check(run.ctx, run.lib.swpc_download_field(run.ctx, field, fptr(b), shape[-1], shape[-2]))
+    assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    run.close()
