@@ -484,15 +484,17 @@ int swpc_fbatch_set_strip(swpc_fbatch *b, int strip_cells);
 /* Launch form of the batch: kernel 0 = the flat one-cell kernels in strip
  * order (swpc_fbatch_set_strip); kernel 5 / 6 = the TMA-staged stress /
  * velocity kernels with tile (bi, bj) and mpc members per CTA, whose CTAs copy
- * the medium of a tile once for the mpc members (FP32 contexts; the default,
- * stress (4,2) and velocity (4,2) with 2 members per CTA).  Compiled stress
+ * the medium of a tile once for the mpc members (FP32 contexts; the default:
+ * one member per CTA, tiles fastest, both phases on (4,2) tiles below 6,000
+ * tiles of four planes over all members and on (4,4) from there).  Compiled stress
  * (bi, bj, mpc): (4,4,1) (2,4,1) (4,2,1) (4,2,2) (2,4,2) (2,2,2) (2,2,4)
  * (4,1,4); velocity: (4,2,1) (4,4,1) (2,2,1) (4,2,2) (2,2,2) (4,1,2) (2,2,4)
  * (4,1,4).  kernel 7 sets the staged launch order: mpc = 0 member groups
  * fastest (the medium of a tile is re-read from L2), 1 tiles fastest (the
  * halos of neighbouring tiles are).  swpc_fbatch_autotune tunes the form in
  * use (strip widths, or the staged order and the shapes of stress then
- * velocity); swpc_fbatch_get_launch writes {staged, strip, stress bi, bj,
+ * velocity; the form in use stays unless another is faster);
+ * swpc_fbatch_get_launch writes {staged, strip, stress bi, bj,
  * mpc, velocity bi, bj, mpc, tiles first} to out[9]. */
 int swpc_fbatch_set_launch(swpc_fbatch *b, int kernel, int mpc, int bi, int bj);
 int swpc_fbatch_get_launch(const swpc_fbatch *b, int *out);
@@ -603,8 +605,9 @@ long long swpc_device_bytes(const swpc_ctx *ctx);
  * memory by bulk tensor copies; minb must be 1, and the compiled tiles
  * (bi, bj) are stress (4,4) (2,4) (4,2), velocity (4,4) (4,2) (2,2); the
  * reduced storage forms (BF16_R, F16_SR) compile (4,4) and (4,2) for both.
- * 3D contexts start with kernels 5 (4,4) and 6 (4,4); the reduced storage
- * forms with kernel 5 on (4,2).
+ * 3D contexts start with kernels 5 and 6, on (4,2) tiles below 6,000 tiles of
+ * four planes and on (4,4) from there; the reduced storage forms with kernel 5
+ * on (4,2) and 6 on (4,4).
  * kernel 7 (3D) sets the launch order of the staged kernels: tiles run k
  * fastest, then over (i, j) in blocks of bi consecutive j tiles (j fastest
  * within a block), so that a tile's j-halo is still in L2; bi = 1 runs i then
@@ -621,7 +624,7 @@ long long swpc_device_bytes(const swpc_ctx *ctx);
  * 2D contexts (P-SV, SH) take kernels 0 / 1 (the tile-walking stress /
  * velocity kernels) and 5 / 6 (the staged ones: a CTA per 32 x 16 tile with
  * bi = 4, 8 or 16 threads along i, minb 1, bj 1); they start with kernels
- * 5 and 6 at bi = 8.
+ * 5 and 6 at bi = 16 up to 444 tiles (three per SM) and at bi = 8 beyond.
  * The defaults come from sweeps on B200.  No counterpart in the reference
  * (its OpenMP/OpenACC schedules are fixed at compile time); results are
  * bitwise independent of the variant. */

@@ -1573,8 +1573,8 @@ static int build_graph(swpc_ctx *c, int steps, cudaGraphExec_t *exec) {
 
 // Steps per graph.  One graph launch costs the host about 7 us, as much as a
 // small grid's step takes on the GPU, and no launch overlaps the end of the
-// graph before it: grids whose step is short replay several steps at a time
-// (reports come every multiple of ten steps).  With ten steps against one: a
+// graph before it: grids whose step is short replay ten steps at a time, and
+// what a call of swpc_run leaves over one by one.  With ten steps against one: a
 // 40 x 36 x 32 shot 1.31 against 1.45 ms, 300 steps of a 256 x 128 P-SV model
 // 3.12 against 3.90 ms, 200 steps of a 517 x 259 SH model 1.88 against 2.32 ms.
 // A step of a million cells takes over 40 us, and the launches of one step per

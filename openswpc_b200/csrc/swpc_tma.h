@@ -7,10 +7,11 @@
 
 namespace swpc {
 
-// Division of a CTA index by a launch constant as a multiply and a shift (exact
-// for 0 <= n < 2^31; m = floor(2^32 (2^s - d) / d) + 1 with 2^s the first power
-// of two >= d): the lead thread of a tile divides four times before it can
-// issue its copies.
+// Division of a CTA index by a launch constant as a multiply and a shift
+// (Granlund and Montgomery, Division by invariant integers using
+// multiplication, 1994; exact for 0 <= n < 2^31; m = floor(2^32 (2^s - d) / d)
+// + 1 with 2^s the first power of two >= d): the lead thread of a tile divides
+// four times before it can issue its copies.
 struct FastDiv {
     unsigned d, m, s;
     static FastDiv of(int n) {
